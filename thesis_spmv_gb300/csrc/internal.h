@@ -101,6 +101,48 @@ cudaError_t launch_sell_spmv(const SellPlan& S, bool bf16, const int32_t* row_st
                              const double* nsq_in, double* nsq_out, unsigned int* counter, int sm_count,
                              cudaStream_t st);
 
+// diag.cu: diagonal slices (64 rows; per slot one column - row offset, a row
+// mask and the rows' values) of a matrix whose entries lie on few diagonals;
+// the FP64 SpMV and power steps, and the FP32 / BF16 ones, of stencils.
+struct DiagPlan {
+    int nslices = 0;             // 0: the matrix does not fit the layout
+    long long elems = 0;         // stored elements (64 per slot)
+    void* mem = nullptr;         // the allocation that rec .. val64 and npart lie in
+    int2* rec = nullptr;         // per slice: {first slot, slots << 1 | some slot lacks rows}
+    int32_t* offs = nullptr;     // per slot: column - row
+    void* masks = nullptr;       // per slot: the rows of the slice that have an element
+    double* val64 = nullptr;     // value of row 32 r + l of the slice at (slot * 32 + l) * 2 + r
+    float* val32 = nullptr;      // the same in FP32 (made on first use)
+    void* valbf = nullptr;       // the same in BF16 (made on first use)
+    double* npart = nullptr;     // per-CTA shares of ||y||^2
+    void release();
+};
+// 0 = built, 1 = the matrix does not fit (D stays empty), 2 = a CUDA error or
+// no memory (D stays empty).
+int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
+               int sm_count, cudaStream_t st);
+int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st);
+// One pass over slices [c0, c1) (c1 < 0: all).  mode kModeSpmv: y = A x;
+// kModePower: y = 2^e A x and *nsq_out = ||y||^2 (when given; counter zero
+// between launches); kModeScale: y = 2^e A x and atomicMax(*mx_out) of y's
+// magnitude keys.  e from *mx_in, else *nsq_in, else 0.
+struct DiagStep {
+    const unsigned int* mx_in = nullptr;
+    const double* nsq_in = nullptr;
+    unsigned int* mx_out = nullptr;
+    unsigned int* counter = nullptr;
+    double* nsq_out = nullptr;
+    int c0 = 0, c1 = -1;
+    bool pdl = true;
+};
+cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, int noc, const void* x, void* y,
+                             const DiagStep& s, int sm_count, cudaStream_t st);
+// Pipelined host-array SpMV: out[p] = the largest column the slices of chunks
+// 0..p read (slices [0, nslices (p + 1) / K)).
+cudaError_t launch_diag_maxcol(const DiagPlan& D, int nor, int noc, int K, int* out, cudaStream_t st);
+int diag_slice_rows();
+void diag_warm_launch_caches();
+
 // l1: launch variant of the merge kernels.  Bit 0: 0 = most resident CTAs,
 // 1 = a smaller shared-memory carveout, more L1 for irregular gathers; bit 1:
 // stream the plan's 16-bit column offsets (set only when the plan has them);

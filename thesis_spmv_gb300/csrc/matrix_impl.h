@@ -98,6 +98,8 @@ struct pwmgpu_matrix {
     // may use it (PWMGPU_LOWFMT_*)
     pwmgpu::SellPlan sell;
     int low_format = PWMGPU_LOWFMT_AUTO;
+    // diagonal slices (nslices 0: the matrix does not fit them)
+    pwmgpu::DiagPlan diag;
 
     // scratch
     double* carries = nullptr;  // max(num_tiles, num_tiles32) doubles (also used as floats)
@@ -205,6 +207,7 @@ struct pwmgpu_matrix {
         valbf = nullptr;
         bf16_exact = -1;
         sell.release();
+        diag.release();
         M = DevMatrix();
         num_tiles = 0;
         loaded = false;

@@ -1111,6 +1111,7 @@ void warm_launch_caches(int sm_count) {
             (void)power_persistent_grid(cfg, 1, sm_count, v);
         }
     (void)sell_grid(1, sm_count);
+    diag_warm_launch_caches();
 }
 
 int merge_grid(int cfg, int nsub, int sm_count, int l1) {

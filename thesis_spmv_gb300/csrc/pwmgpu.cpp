@@ -200,11 +200,15 @@ int tune(pwmgpu_matrix* m) {
     // variants: carveout (bit 0) x gathers through L1 or around it (bit 2)
     const int cand[4] = {0, 1, 4, 5};
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
+    // a matrix on diagonal slices runs the merge kernels only where the handle
+    // asks for them: two timed runs do (36 -> 12 SpMVs, 1.4 ms of the load of
+    // a 2048^2 stencil)
+    const int reps = m->diag.nslices ? 2 : 8;
     for (int c = 0; c < 4 && rc == PWMGPU_OK; ++c) {
         const int v = cand[c] | c16;
         const int grid = merge_grid(kCfgF64, m->num_tiles, m->sm_count, v);
         cudaError_t e = cudaSuccess;
-        for (int r = 0; r < 9 && e == cudaSuccess; ++r) {  // one warm-up, eight timed
+        for (int r = 0; r <= reps && e == cudaSuccess; ++r) {  // one warm-up, the rest timed
             if (r == 1) e = cudaEventRecord(e0, m->stream);
             if (e == cudaSuccess)
                 e = launch_merge_spmv(kCfgF64, kModeSpmv, m->M, m->P.valp, m->P, grid, m->dx, m->dy, m->carries,
@@ -214,7 +218,7 @@ int tune(pwmgpu_matrix* m) {
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[c], e0, e1);
         if (e != cudaSuccess) rc = fail(PWMGPU_ERR_CUDA, "launch tuning: %s", cudaGetErrorString(e));
-        ms[c] /= 8.f;
+        ms[c] /= (float)reps;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -291,6 +295,10 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
     TRY(build_col16(m));
     // fix-up descriptors; without them (no memory) the search-based fix-up runs
     (void)build_fix_runs(m->P, m->M.row_start, m->M.nor, m->sm_count, m->stream);
+    // diagonal slices where the matrix fits them (no memory: the merge plan
+    // alone); the serving loop's batched kernels do not read them
+    if (!m->skip_tune)
+        (void)diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count, m->stream);
     dfree(m->M.col);
     dfree(m->M.val);
     m->l1 = m->P.colp16 ? 2 : 0;
@@ -425,6 +433,10 @@ int fp64_format(const pwmgpu_matrix* m) {
 int spmv_f64(pwmgpu_matrix* m, const double* dx, double* dy) {
     if (fp64_format(m) != PWMGPU_FMT_MERGE) return spmv_format(m, fp64_format(m), dx, dy, nullptr);
     if (m->num_tiles == 0) return PWMGPU_OK;
+    if (m->diag.nslices) {
+        CU(launch_diag_spmv(m->diag, kCfgF64, kModeSpmv, m->M.nor, m->M.noc, dx, dy, DiagStep{}, m->sm_count, m->stream));
+        return PWMGPU_OK;
+    }
     CU(launch_merge_spmv(kCfgF64, kModeSpmv, m->M, m->P.valp, m->P, m->grid, dx, dy, m->carries, nullptr, m->status,
                          m->stream, m->l1));
     if (m->P.runs)
@@ -447,6 +459,15 @@ bool norm_in_step(const pwmgpu_matrix* m, int grid) {
 // descriptors.
 int power_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double* nsq_in, double* nsq_out,
                    const unsigned int* mx_in = nullptr) {
+    if (m->diag.nslices) {
+        DiagStep s;
+        s.mx_in = mx_in;
+        s.nsq_in = nsq_in;
+        s.counter = m->counter + 2;
+        s.nsq_out = nsq_out;
+        CU(launch_diag_spmv(m->diag, kCfgF64, kModePower, m->M.nor, m->M.noc, in, out, s, m->sm_count, m->stream));
+        return PWMGPU_OK;
+    }
     if (norm_in_step(m, m->grid)) {
         CU(launch_merge_spmv(kCfgF64, kModePower, m->M, m->P.valp, m->P, m->grid, in, out, m->carries, nsq_in,
                              m->status, m->stream, m->l1, m->npart, mx_in));
@@ -476,6 +497,14 @@ int power_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double
 // Needs the plan's run descriptors (norm_in_step).
 int scale_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double* nsq_in, const unsigned int* mx_in,
                    unsigned int* mx_out) {
+    if (m->diag.nslices) {
+        DiagStep s;
+        s.mx_in = mx_in;
+        s.nsq_in = nsq_in;
+        s.mx_out = mx_out;
+        CU(launch_diag_spmv(m->diag, kCfgF64, kModeScale, m->M.nor, m->M.noc, in, out, s, m->sm_count, m->stream));
+        return PWMGPU_OK;
+    }
     CU(launch_merge_spmv(kCfgF64, kModeScale, m->M, m->P.valp, m->P, m->grid, in, out, m->carries, nsq_in,
                          m->status, m->stream, m->l1, nullptr, mx_in, mx_out));
     CU(launch_fix_runs_scale(false, m->P, out, m->carries, nsq_in, mx_in, mx_out, m->stream));
@@ -523,7 +552,7 @@ int power_device(pwmgpu_matrix* m, double* dx, double* dy, int32_t it) {
         // The last two steps compute the exact norms the final normalisation
         // uses; the steps before them only need the rescale exponent, from
         // their input's largest magnitude key (MODE_SCALE).
-        const bool scale = norm_in_step(m, m->grid);
+        const bool scale = m->diag.nslices || norm_in_step(m, m->grid);
         if (scale) TRY(ensure_mxk(m, (size_t)it + 1));
         for (int k = 0; k < it; ++k) {
             const double* in = (k % 2 == 0) ? dx : dy;
@@ -548,18 +577,25 @@ int power_device(pwmgpu_matrix* m, double* dx, double* dy, int32_t it) {
 // Poisson 4 / -1 stencil is) BF16 copy of the values, made on first use.
 }  // namespace
 namespace pwmgpu {
+namespace {
+// m->bf16_exact: whether every value is exactly a BF16 number.
+int ensure_bf16_exact(pwmgpu_matrix* m) {
+    if (m->bf16_exact >= 0) return PWMGPU_OK;
+    int* flag = reinterpret_cast<int*>(m->barrier + 2);
+    int h = 0;
+    CU(cudaMemsetAsync(flag, 0, sizeof(int), m->stream));
+    CU(launch_bf16_exact(m->P.valp, mli_storage_elems(m->M.nnz, m->P.nsub), flag, m->sm_count, m->stream));
+    CU(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+    CU(cudaStreamSynchronize(m->stream));
+    m->bf16_exact = h == 0 ? 1 : 0;
+    return PWMGPU_OK;
+}
+}  // namespace
+
 int ensure_low_values(pwmgpu_matrix* m, bool allow_bf16, int* cfg, const void** valp, int* pgrid) {
     const long long elems = mli_storage_elems(m->M.nnz, m->P.nsub);
     if (allow_bf16) {
-        if (m->bf16_exact < 0) {
-            int* flag = reinterpret_cast<int*>(m->barrier + 2);
-            int h = 0;
-            CU(cudaMemsetAsync(flag, 0, sizeof(int), m->stream));
-            CU(launch_bf16_exact(m->P.valp, elems, flag, m->sm_count, m->stream));
-            CU(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-            CU(cudaStreamSynchronize(m->stream));
-            m->bf16_exact = h == 0 ? 1 : 0;
-        }
+        TRY(ensure_bf16_exact(m));
         if (m->bf16_exact == 1) {
             if (!m->valbf) {
                 CU(cudaMalloc(&m->valbf, 2 * (size_t)elems + 16));
@@ -581,6 +617,17 @@ int ensure_low_values(pwmgpu_matrix* m, bool allow_bf16, int* cfg, const void** 
     *valp = m->val32;
     *pgrid = m->pgrid32;
     return PWMGPU_OK;
+}
+
+// Whether iterations of configuration cfg run on the diagonal slices: the
+// matrix fits them, and the handle asks for neither the persistent merge
+// kernel nor (FP32 / BF16) the merge layout.  Makes the FP32 / BF16 values on
+// first use.
+bool diag_for(pwmgpu_matrix* m, int cfg) {
+    if (!m->diag.nslices || m->power_mode == PWMGPU_POWER_FUSED) return false;
+    if (cfg == kCfgF64) return true;
+    return m->low_format == PWMGPU_LOWFMT_AUTO &&
+           diag_low_values(m->diag, cfg == kCfgBF16, m->sm_count, m->stream) == 0;
 }
 
 // The SELL-32 copy with values of configuration cfg (FP32 or BF16), built on
@@ -646,7 +693,38 @@ struct ChunkOut {
 // differs.
 int solve_chunk(pwmgpu_matrix* m, int cfg, const void* valp, int pgrid, void* X, void* Y, int k0, int nk,
                 ChunkOut* o) {
-    if (sell_for(m, cfg)) {
+    if (diag_for(m, cfg)) {
+        // diagonal slices: one kernel per step; the steps before the last
+        // two track only the rescale's magnitude keys, the last one takes
+        // the row pass for v_k . v_{k+1}
+        const bool f32 = cfg != kCfgF64;
+        const int dg = dot_grid(m->M.nor, m->sm_count);
+        if (nk > 2) TRY(ensure_mxk(m, (size_t)(k0 + nk) + 1));
+        for (int k = k0; k < k0 + nk; ++k) {
+            const void* in = (k & 1) ? Y : X;
+            void* out = (k & 1) ? X : Y;
+            const bool keys = k < k0 + nk - 2, last = k == k0 + nk - 1;
+            DiagStep s;
+            if (k > k0 && k - 1 < k0 + nk - 2) s.mx_in = m->mxk + k;
+            else if (k > 0) s.nsq_in = m->nsq + k;
+            s.counter = m->counter + 2;
+            if (keys) s.mx_out = m->mxk + k + 1;
+            else if (!last) s.nsq_out = m->nsq + k + 1;
+            CU(launch_diag_spmv(m->diag, cfg, keys ? kModeScale : kModePower, m->M.nor, m->M.noc, in, out, s,
+                                m->sm_count, m->stream));
+        }
+        const int k = k0 + nk - 1;
+        const void* in = (k & 1) ? Y : X;
+        const void* out = (k & 1) ? X : Y;
+        if (f32)
+            CU(launch_power_norm_f32((const float*)out, (const float*)in, m->M.nor, m->partials, m->counter,
+                                     m->small + 6, dg, m->stream));
+        else
+            CU(launch_power_norm_f64((const double*)out, (const double*)in, m->M.nor, m->partials, m->counter,
+                                     m->small + 6, dg, m->stream));
+        CU(launch_solve_result(f32, in, out, m->M.nor, m->nsq + k, m->small + 6, m->nsq + k + 1, m->small,
+                               m->partials, m->counter, dg, m->stream));
+    } else if (sell_for(m, cfg)) {
         // SELL-32: one kernel per step (no fix-up; ||y||^2 summed in it), the
         // chunk's last step with the norm pass for the Rayleigh dot
         const bool bf = cfg == kCfgBF16;
@@ -774,7 +852,16 @@ int solve(pwmgpu_matrix* m, double* x, int32_t max_it, double tol, int precision
     if (precision == PWMGPU_PREC_F32 || (precision == PWMGPU_PREC_MIXED && budget >= 2)) {
         int cfg = kCfgF32, pg = 0;
         const void* valp = nullptr;
-        TRY(ensure_low_values(m, precision == PWMGPU_PREC_MIXED, &cfg, &valp, &pg));
+        pg = m->pgrid32;
+        if (precision == PWMGPU_PREC_MIXED) {
+            TRY(ensure_bf16_exact(m));
+            if (m->bf16_exact == 1) {
+                cfg = kCfgBF16;
+                pg = m->pgridbf;
+            }
+        }
+        // (diagonal slices hold their own FP32 / BF16 values)
+        if (!diag_for(m, cfg)) TRY(ensure_low_values(m, precision == PWMGPU_PREC_MIXED, &cfg, &valp, &pg));
         if (pg == 0 && m->power_mode == PWMGPU_POWER_FUSED)
             return fail(PWMGPU_ERR_UNSUPPORTED, "the fused power kernel cannot be made co-resident");
         TRY(ensure_fvectors(m));
@@ -865,19 +952,29 @@ int plan_pipeline(pwmgpu_matrix* m) {
     int* d = nullptr;
     TRY(dalloc(&d, 4 * (size_t)K));
     p.rec.assign(4 * (size_t)K, 0);
-    cudaError_t e = launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
+    const bool diag = m->diag.nslices > 0;
+    cudaError_t e = diag ? launch_diag_maxcol(m->diag, m->M.nor, m->M.noc, K, d, m->stream)
+                         : launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(p.rec.data(), d, sizeof(int) * 4 * K, cudaMemcpyDeviceToHost, m->stream);
+        e = cudaMemcpyAsync(p.rec.data(), d, sizeof(int) * (diag ? 1 : 4) * K, cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     dfree(d);
     if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "pipeline plan: %s", cudaGetErrorString(e));
+    // diagonal slices: a chunk is a range of slices, its rows its own
+    if (diag)
+        for (int c = K - 1; c >= 0; --c) {
+            const int s0 = (int)((long long)m->diag.nslices * c / K);
+            const int mx = p.rec[(size_t)c];
+            const int rec[4] = {s0, s0 * diag_slice_rows(), 0, mx};
+            std::copy(rec, rec + 4, p.rec.begin() + 4 * c);
+        }
     // a run of sub-tiles may cross at most one chunk boundary: chunk first
     // rows must increase strictly
     for (int c = 1; c < K; ++c)
         if (p.rec[4 * c + 1] <= p.rec[4 * (c - 1) + 1]) return PWMGPU_OK;
     for (int c = 1; c < K; ++c) p.rec[4 * c + 3] = std::max(p.rec[4 * c + 3], p.rec[4 * (c - 1) + 3]);
     p.fpre.assign(K + 1, 0);
-    if (m->P.runs) {
+    if (m->P.runs && !diag) {
         for (int c = 0; c < K; ++c)
             CU(cudaMemcpy(&p.fpre[(size_t)c], m->P.run_pre + p.rec[4 * c], sizeof(int), cudaMemcpyDeviceToHost));
         p.fpre[(size_t)K] = m->P.nruns;
@@ -922,7 +1019,9 @@ bool sm_reachable_pageable(pwmgpu_matrix* m, const void* h) {
 
 int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
     auto& p = m->pipe;
-    const int K = p.K, noc = m->M.noc, nor = m->M.nor, nsub = m->num_tiles;
+    const int K = p.K, noc = m->M.noc, nor = m->M.nor;
+    const bool diag = m->diag.nslices > 0;
+    const int nsub = diag ? m->diag.nslices : m->num_tiles;
     const bool x_sm = sm_reachable_pageable(m, x), y_sm = sm_reachable_pageable(m, y);
     // the streams start after earlier work on the handle's stream
     CU(cudaEventRecord(p.ev_start, m->stream));
@@ -955,23 +1054,34 @@ int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
             waited = std::max(waited, need);
             int t0, t1;
             chunk_tiles(c, &t0, &t1);
-            const int grid = merge_grid(kCfgF64, t1 - t0, m->sm_count, m->l1);
-            CU(launch_merge_spmv_range(m->M, m->P, t0, t1, grid, m->dx, m->dy, m->carries, m->status, m->stream,
-                                       m->l1));
+            if (diag) {
+                DiagStep s;
+                s.c0 = t0;
+                s.c1 = t1;
+                s.pdl = false;  // as launch_merge_spmv_range
+                CU(launch_diag_spmv(m->diag, kCfgF64, kModeSpmv, nor, noc, m->dx, m->dy, s, m->sm_count, m->stream));
+            } else {
+                const int grid = merge_grid(kCfgF64, t1 - t0, m->sm_count, m->l1);
+                CU(launch_merge_spmv_range(m->M, m->P, t0, t1, grid, m->dx, m->dy, m->carries, m->status, m->stream,
+                                           m->l1));
+            }
         }
-        if (c >= 1) {
-            // chunk c-1: fix-up of its runs (they end by chunk c), then its rows go down
+        // chunk f is done: its rows go down -- the chunk just launched (diagonal
+        // slices), or the one before it after the fix-up of its runs (they end
+        // by chunk c)
+        const int f = diag ? c : c - 1;
+        if (f >= 0 && f < K) {
             int t0, t1;
-            chunk_tiles(c - 1, &t0, &t1);
-            if (m->P.runs)
-                CU(launch_fix_runs_f64(kModeSpmv, m->P, p.fpre[(size_t)c - 1], p.fpre[(size_t)c], m->dy, m->carries,
+            chunk_tiles(f, &t0, &t1);
+            if (!diag && m->P.runs)
+                CU(launch_fix_runs_f64(kModeSpmv, m->P, p.fpre[(size_t)f], p.fpre[(size_t)f + 1], m->dy, m->carries,
                                        nullptr, m->stream));
-            else
+            else if (!diag)
                 CU(launch_merge_fixup_range(m->M, m->P.subc, nsub, t0, t1, m->dy, m->carries, m->stream,
                                             m->sm_count));
-            CU(cudaEventRecord(p.ev_y[(size_t)c - 1], m->stream));
-            CU(cudaStreamWaitEvent(p.out, p.ev_y[(size_t)c - 1], 0));
-            const int r0 = row_lo(c - 1), r1 = row_lo(c);
+            CU(cudaEventRecord(p.ev_y[(size_t)f], m->stream));
+            CU(cudaStreamWaitEvent(p.out, p.ev_y[(size_t)f], 0));
+            const int r0 = row_lo(f), r1 = row_lo(f + 1);
             if (r1 > r0 && y_sm)
                 CU(launch_host_copy(m->dy + r0, y + r0, r1 - r0, p.out));
             else if (r1 > r0)
@@ -1501,6 +1611,11 @@ int pwmgpu_mv_device_f32(pwmgpu_matrix* m, const float* dx, float* dy) {
     if (m->format != PWMGPU_FMT_MERGE) return fail(PWMGPU_ERR_UNSUPPORTED, "FP32 SpMV runs on the merge format");
     if (m->M.nor > 0 && (!dx || !dy)) return fail(PWMGPU_ERR_INVALID, "null vector");
     if (m->num_tiles == 0) return PWMGPU_OK;
+    if (diag_for(m, kCfgF32)) {
+        CU(launch_diag_spmv(m->diag, kCfgF32, kModeSpmv, m->M.nor, m->M.noc, dx, dy, DiagStep{}, m->sm_count,
+                            m->stream));
+        return PWMGPU_OK;
+    }
     if (sell_for(m, kCfgF32)) {
         CU(launch_sell_spmv(m->sell, false, m->M.row_start, m->M.nor, dx, dy, nullptr, nullptr, m->counter + 2,
                             m->sm_count, m->stream));
