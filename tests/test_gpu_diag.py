@@ -128,3 +128,45 @@ def test_a_handle_reloaded_with_another_kind(pwm):
         y = np.zeros(A.nor)
         M.mv(x, y)
         assert np.all(np.abs(y - O.crs_mv(A, x)) <= O.row_error_bound(A, x))
+
+
+@pytest.mark.parametrize("steps,graph", [(2, True), (3, True), (4, False), (8, True)])
+def test_service_batches(pwm, steps, graph):
+    """The serving loop's diagonal-slice classes: matrices of 1 .. 300 slices,
+    3 .. 11 slots, in every precision, beside one that does not fit the
+    layout.  Rounds of 2 and 3 steps have no or one key step.  Each solve's
+    eigenpair against the oracle, and the same bits alone as in the mix."""
+    from thesis_spmv_gb300.service import Service
+    mats = []
+    for k, (n, offs) in enumerate([(40, [-1, 0, 1]), (64, [-8, -1, 0, 1, 8]), (1000, range(-5, 6)),
+                                   (19000, [-137, -1, 0, 1, 137])]):
+        A = _diagonals(n, n, offs, 40 + k)
+        A.data = np.abs(A.data) + 0.05
+        mid = A.row_start[n // 2] + int(np.argmin(np.abs(A.col_ind[A.row_start[n // 2]:A.row_start[n // 2 + 1]] - n // 2)))
+        A.data[mid] += 12.0  # a dominant, well separated eigenvalue
+        mats.append(A)
+    rng = np.random.default_rng(7)
+    n = 800
+    cols = np.sort(np.argsort(rng.random((n, n)), axis=1)[:, :6], axis=1).astype(np.int32)
+    mats.append(O.CRSArrays(n, n, (6 * np.arange(n + 1)).astype(np.int32), cols.reshape(-1), rng.uniform(0.1, 1, 6 * n)))
+
+    def run(which):
+        svc = Service(hbm_budget_bytes=1 << 30, round_iterations=steps, use_graph=graph)
+        ids = []
+        for i, prec in which:
+            x0 = np.random.default_rng(100 + i).random(mats[i].nor)
+            tol = 1e-5 if prec == pwm.PREC_F32 else 1e-10
+            ids.append(svc.submit_csr(mats[i], max_it=6000, tol=tol, precision=prec, x0=x0, keep_vector=True))
+        svc.run_until_idle()
+        return [svc.result(i, want_vector=True) for i in ids]
+
+    which = [(i, p) for i in range(len(mats)) for p in (pwm.PREC_F64, pwm.PREC_F32, pwm.PREC_MIXED)]
+    for (i, prec), (r, u) in zip(which, run(which)):
+        assert r.converged == 1
+        lam, res = O.rayleigh(mats[i], u)
+        assert res <= (1e-4 if prec == pwm.PREC_F32 else 2e-10)
+        assert abs(r.lambda_ - lam) <= (1e-5 if prec == pwm.PREC_F32 else 1e-10) * abs(lam)
+        if i in (0, 3):
+            (ra, ua), = run([(i, prec)])
+            assert ra.iterations == r.iterations and ra.lambda_ == r.lambda_
+            assert np.array_equal(ua.view(np.uint64), u.view(np.uint64))

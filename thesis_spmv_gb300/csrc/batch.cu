@@ -44,10 +44,23 @@ __device__ __forceinline__ int find_slot(const BatchSlot* __restrict__ slots, in
     int lo = 0, hi = nslots - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        const int key = FIELD == 0 ? __ldg(&slots[mid].tile0) : FIELD == 1 ? __ldg(&slots[mid].fix0)
-                                                                            : __ldg(&slots[mid].row0);
+        const int key = FIELD == 0 ? __ldg(&slots[mid].tile0) : __ldg(&slots[mid].fix0);
         if (key <= v) lo = mid;
         else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The slot of row chunk c, found by the calling warp's lanes together (32
+// ways per step: two dependent loads for 1024 slots).
+__device__ __forceinline__ int find_row_slot(const BatchSlot* __restrict__ slots, int nslots, int c) {
+    int lo = 0, n = nslots;  // the slot lies in [lo, lo + n)
+    while (n > 1) {
+        const int step = (n + 31) >> 5, at = lo + (int)(threadIdx.x & 31) * step;
+        const bool ok = at < lo + n && __ldg(&slots[at].row0) <= c;  // lanes 0 .. some l
+        const int l = 31 - __clz(__ballot_sync(0xffffffffu, ok));
+        n = min(step, lo + n - (lo + l * step));
+        lo += l * step;
     }
     return lo;
 }
@@ -436,20 +449,23 @@ __device__ __forceinline__ void chunk_sums(const XT* __restrict__ y, const XT* _
     if (DOT) dd += ((d[0] + d[1]) + (d[2] + d[3])) + dr;
 }
 
+// ahead: steps done since the state's k last advanced (a diagonal-slice
+// round's key steps; 0 in the other classes).
 template <typename XT>
-__global__ void __launch_bounds__(256, 3) k_batch_norm(const BatchTable* __restrict__ Tp, int want_dot) {
+__global__ void __launch_bounds__(256, 3) k_batch_norm(const BatchTable* __restrict__ Tp, int want_dot, int ahead) {
     __shared__ double red[32];
     __shared__ int last;
     const BatchTable T = *Tp;
+    pdl_wait();
     for (int c = blockIdx.x; c < T.nrow; c += gridDim.x) {
-        const int j = find_slot<2>(T.slots, T.nslots, c);
+        const int j = find_row_slot(T.slots, T.nslots, c);
         const BatchSlot& d = T.slots[j];
         SlotState* stt = T.states + d.state;
-        const int kit = stt->k;
+        const int kit = stt->k + ahead;
         const XT* in = static_cast<const XT*>((kit & 1) ? d.Y : d.X);
         const XT* out = static_cast<const XT*>((kit & 1) ? d.X : d.Y);
-        const int lo = (c - d.row0) * kRowChunk;
-        const int hi = min(d.nor, lo + kRowChunk);
+        const int lo = (c - d.row0) * d.rchunk;
+        const int hi = min(d.nor, lo + d.rchunk);
         double sq = 0.0, dd = 0.0;
         if (want_dot) chunk_sums<XT, true>(out, in, lo, hi, sq, dd);
         else chunk_sums<XT, false>(out, in, lo, hi, sq, dd);
@@ -476,7 +492,10 @@ __global__ void __launch_bounds__(256, 3) k_batch_norm(const BatchTable* __restr
             if (threadIdx.x == 0) {
                 stt->nsq_prev = stt->nsq;
                 stt->nsq = s0;
-                if (want_dot) stt->dot = s1;
+                if (want_dot) {
+                    stt->dot = s1;
+                    stt->mxr[0] = stt->mxr[1] = stt->mxr[2] = 0u;
+                }
                 stt->keyed = 0;
                 stt->k = kit + 1;
                 stt->norm_count = 0u;
@@ -491,8 +510,9 @@ __global__ void __launch_bounds__(256) k_batch_resid(const BatchTable* __restric
     __shared__ double red[32];
     __shared__ int last;
     const BatchTable T = *Tp;
+    pdl_wait();
     for (int c = blockIdx.x; c < T.nrow; c += gridDim.x) {
-        const int j = find_slot<2>(T.slots, T.nslots, c);
+        const int j = find_row_slot(T.slots, T.nslots, c);
         const BatchSlot& d = T.slots[j];
         SlotState* stt = T.states + d.state;
         const int kit = stt->k;  // >= 2 after a round
@@ -518,8 +538,8 @@ __global__ void __launch_bounds__(256) k_batch_resid(const BatchTable* __restric
         }
         const XT* cur = static_cast<const XT*>((kit & 1) ? d.Y : d.X);
         const XT* prev = static_cast<const XT*>((kit & 1) ? d.X : d.Y);
-        const int lo = (c - d.row0) * kRowChunk;
-        const int hi = min(d.nor, lo + kRowChunk);
+        const int lo = (c - d.row0) * d.rchunk;
+        const int hi = min(d.nor, lo + d.rchunk);
         double rr = 0.0;
         for (int r = lo + threadIdx.x; r < hi; r += blockDim.x) {
             const double dl = scale_pow2((double)__ldcg(cur + r), -e) - lam * (double)__ldcg(prev + r);
@@ -588,7 +608,7 @@ struct BatchKernels {
         }
         k_batch_spmv<VT, XT, AT, kBatchNT, kMliIpt><<<grid<false>(sm_count), kBatchNT, SMEM, st>>>(T);
         k_batch_fixup<XT, AT><<<8 * sm_count, 256, 0, st>>>(T);
-        k_batch_norm<XT><<<3 * sm_count, 256, 0, st>>>(T, want_dot);
+        k_batch_norm<XT><<<3 * sm_count, 256, 0, st>>>(T, want_dot, 0);
         return cudaGetLastError();
     }
 };
@@ -623,7 +643,7 @@ static void launch_batch_sell(const BatchTable* T, int sum, int sm_count, cudaSt
         k_batch_grp<<<sm_count, 256, 0, st>>>(T);
     } else {
         k_batch_sell<VT, kSellNone><<<sell_batch_grid<VT, kSellNone>(sm_count), 256, 0, st>>>(T);
-        k_batch_norm<float><<<3 * sm_count, 256, 0, st>>>(T, 1);
+        k_batch_norm<float><<<3 * sm_count, 256, 0, st>>>(T, 1, 0);
     }
 }
 
@@ -634,6 +654,7 @@ void batch_prepare(int sm_count) {
     BatchKernels<float, float, float>::grid<true>(sm_count);
     BatchKernels<__nv_bfloat16, float, float>::grid<false>(sm_count);
     BatchKernels<__nv_bfloat16, float, float>::grid<true>(sm_count);
+    batch_diag_prepare(sm_count);
     sell_batch_grid<float, kSellNone>(sm_count);
     sell_batch_grid<float, kSellSquares>(sm_count);
     sell_batch_grid<float, kSellKeys>(sm_count);
@@ -642,10 +663,44 @@ void batch_prepare(int sm_count) {
     sell_batch_grid<__nv_bfloat16, kSellKeys>(sm_count);
 }
 
+// A row pass launched so that it may start while the kernel before it on the
+// stream ends (it waits for it before its first read).
+template <typename... A>
+static cudaError_t launch_after(void (*k)(A...), int grid, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+// A diagonal-slice class's round: one kernel per step, the norm pass after
+// the last two, the residual.
+template <typename XT>
+static cudaError_t batch_diag_round(int cfg, const BatchTable* T, int steps, int sm_count, cudaStream_t st) {
+    for (int it = 0; it < steps; ++it) {
+        const bool keys = it < steps - 2, last = it == steps - 1;
+        cudaError_t e = launch_batch_diag(cfg, T, it, keys, it > 0 && !last, sm_count, st);
+        if (e == cudaSuccess && !keys)
+            e = launch_after(k_batch_norm<XT>, 3 * sm_count, st, T, last ? 1 : 0, last ? 0 : it);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_after(k_batch_resid<XT>, 4 * sm_count, st, T);
+}
+
 // A round of `steps` power steps: key steps, then the two steps whose norms
 // the round's Rayleigh quotient and residual use (||v_{k-1}||^2, then
 // ||v_k||^2 with v_{k-1} . v_k), then the residual.
-cudaError_t launch_batch_round(int cfg, const BatchTable* T, int steps, int sm_count, cudaStream_t st, bool sell) {
+cudaError_t launch_batch_round(int cfg, const BatchTable* T, int steps, int sm_count, cudaStream_t st, int layout) {
+    if (layout == kBatchDiag)
+        return cfg == kCfgF64 ? batch_diag_round<double>(cfg, T, steps, sm_count, st)
+                              : batch_diag_round<float>(cfg, T, steps, sm_count, st);
+    const bool sell = layout == kBatchSell;
     for (int it = 0; it < steps; ++it) {
         const int want_dot = it == steps - 1;
         const bool keys = it < steps - 2;

@@ -19,7 +19,15 @@ namespace pwmgpu {
 
 constexpr int kFixTiles = 256;    // sub-tiles per fix-up chunk (one per thread: a fix-up is latency-bound)
 constexpr int kSellGroup = 16;    // SELL-32 classes: slices per group of the in-kernel norm
-constexpr int kRowChunk = 16384;  // rows per norm / residual chunk (a multiple of 4)
+// Rows per norm / residual chunk (one CTA's work; a multiple of 4) of a solve
+// with nor rows: enough chunks that a few solves spread over the SMs, few
+// enough that the sums over a large one stay a stream.  It depends on the
+// solve alone, so its sums do not depend on the mix.
+constexpr int row_chunk(int nor) {
+    int c = 1024;
+    while (c < 16384 && c < nor / 64) c *= 2;
+    return c;
+}
 
 struct BatchSlot {
     const int32_t* row_start;
@@ -33,13 +41,16 @@ struct BatchSlot {
     void* carries;
     const int32_t* soff;    // SELL-32 classes: slice offsets (nsub = slices, tile0 = first global slice)
     const uint16_t* col16;  // SELL-32 classes: 16-bit column offsets (values in valp)
+    const int2* drec;       // diagonal-slice classes: slice records, offsets and masks (values in valp)
+    const int32_t* doffs;
+    const unsigned* dmasks;
     int nor, nsub;
     int tile0;       // first global sub-tile
     int fix0, nfix;  // fix-up chunks [fix0, fix0 + nfix) (kFixTiles sub-tiles each); SELL-32
                      // classes: slice groups (kSellGroup slices each) of the norm
-    int row0, nrow;  // row chunks [row0, row0 + nrow) (kRowChunk rows each)
+    int row0, nrow;  // row chunks [row0, row0 + nrow) of rchunk rows each
+    int rchunk;      // row_chunk(nor)
     int state;       // index into the state array
-    int pad;
 };
 
 // Per-solve iteration state, advanced on the device.
@@ -58,7 +69,7 @@ struct SlotState {
     unsigned int mx;       // largest magnitude key of v_k (when keyed)
     unsigned int mx_next;  // atomic-max target of a key step (zero between steps)
     int keyed;             // v_k came from a key step: its rescale uses mx, nsq is stale
-    int pad;
+    unsigned int mxr[3];   // diagonal-slice classes: the key words of a round's steps (zero between rounds)
 };
 
 struct BatchTable {

@@ -37,29 +37,13 @@
 #include <algorithm>
 #include <climits>
 
+#include "diag.cuh"
 #include "internal.h"
 #include "merge.cuh"
 
 namespace pwmgpu {
 
 namespace {
-
-// 4 CTAs of 256 threads per SM: 64 registers hold the ten x loads a lane has
-// in flight without a spill, and 160 KB of stages leave 68 KB of L1 for x.
-// (48 registers spill: 0.35 ms on the 4096^2 stencil; 3 CTAs 0.173 ms.)
-constexpr int kDiagNT = 256;
-constexpr int kDiagOcc = 4;
-constexpr int kDiagR = 2;           // rows per lane
-constexpr int kDiagRows = 32 * kDiagR;
-constexpr int kDiagU = 5;           // slots per group (staged, and x loaded, together)
-constexpr int kDiagStages = 2;      // groups staged: the one in use and the next
-constexpr int kDiagMaxSlots = 256;  // per slice: more is no diagonal matrix
-constexpr int kDiagMaxCtas = 8;     // per SM (room for the shares of ||y||^2)
-
-// The rows of a slot that hold an element: bit l of word r for row 32 r + l.
-struct __align__(4 * kDiagR) SlotMask {
-    unsigned w[kDiagR];
-};
 
 // The rows of a slice walked together: head() is the smallest column - row
 // offset among the rows' next elements (INT_MAX: none left); the walk's user
@@ -189,25 +173,6 @@ __global__ void k_diag_convert(const double* __restrict__ in, VT* __restrict__ o
         out[i] = (VT)in[i];
 }
 
-// The lane's values of one slot, global -> shared, asynchronously (read once
-// per pass: evict-first).
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void* dst, const void* src, uint64_t pol) {
-    if (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src),
-                     "l"(pol)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], %2, %3;" ::"r"(smem_u32(dst)), "l"(src),
-                     "n"(BYTES), "l"(pol)
-                     : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copy_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 template <typename VT, typename XT>
 struct DiagArgs {
     const int2* rec;
@@ -225,48 +190,6 @@ struct DiagArgs {
     double* nsq_out;
 };
 
-// A group: the next kDiagU (or fewer) slots of a warp's slice c.  offl and
-// ml: the group's offsets and (where some slot lacks rows) mask words, one
-// per lane, loaded when the group is staged.
-struct Group {
-    int c, slot;
-    int left;  // 2 * slots of the slice from `slot` on + (some slot lacks rows)
-    int offl;
-    unsigned ml;
-};
-
-// At most kDiagU slots: acc[r] += value * x[row + 32 r + offset], in slot
-// order.  All x loads go out together, then the wait for the values.
-template <bool PART, typename VT, typename XT>
-__device__ __forceinline__ void group_fma(const XT* __restrict__ xr, const VT* st, const Group& q, int lane,
-                                          XT (&acc)[kDiagR]) {
-    XT g[kDiagU][kDiagR];
-    const int m = q.left >> 1;
-    unsigned on = ~0u;  // bit u R + r: the lane's row r has an element in slot u
-    if (PART) {
-        on = 0u;
-#pragma unroll
-        for (int i = 0; i < kDiagU * kDiagR; ++i) on |= ((__shfl_sync(0xffffffffu, q.ml, i) >> lane) & 1u) << i;
-    }
-#pragma unroll
-    for (int u = 0; u < kDiagU; ++u) {
-        const XT* xd = xr + __shfl_sync(0xffffffffu, q.offl, u);
-#pragma unroll
-        for (int r = 0; r < kDiagR; ++r)
-            g[u][r] = u < m && (!PART || ((on >> (u * kDiagR + r)) & 1u)) ? __ldg(xd + 32 * r) : XT(0);
-    }
-    copy_wait<kDiagStages - 1>();
-#pragma unroll
-    for (int u = 0; u < kDiagU; ++u) {
-        if (u < m) {
-#pragma unroll
-            for (int r = 0; r < kDiagR; ++r)
-                if (!PART || ((on >> (u * kDiagR + r)) & 1u))
-                    acc[r] = fma((XT)st[u * kDiagRows + r], g[u][r], acc[r]);
-        }
-    }
-}
-
 template <int MODE, typename VT, typename XT>
 __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -283,14 +206,11 @@ __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT
     int ps = prec.x, pl = prec.y;
     prec = pc + tw < a.c1 ? __ldg(a.rec + pc + tw) : make_int2(0, 0);
     auto stage_next = [&](int stage) {
-        Group q{pc, ps, pl, 0, 0u};
+        DiagGroup q{pc, ps, pl, 0, 0u};
         if (pc < a.c1) {
             const int m = pl >> 1;
             const VT* src = a.val + ((size_t)ps * kDiagRows + lane * kDiagR);
-            VT* dst = ring + stage * (kDiagU * kDiagRows);
-#pragma unroll
-            for (int u = 0; u < kDiagU; ++u)
-                if (u < m) copy_async<kDiagR * (int)sizeof(VT)>(dst + u * kDiagRows, src + u * kDiagRows, pol);
+            stage_group(ring + stage * (kDiagU * kDiagRows), src, m, pol);
             if (lane < m) q.offl = __ldg(a.offs + ps + lane);
             if ((pl & 1) && lane < m * kDiagR) q.ml = __ldg(a.masks + (size_t)ps * kDiagR + lane);
             ps += kDiagU;
@@ -306,7 +226,7 @@ __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT
         return q;
     };
     // plan data: loaded before the kernel before on the stream has ended
-    Group cur = stage_next(0);
+    DiagGroup cur = stage_next(0);
     pdl_wait();
     int e = 0;
     if (MODE != MODE_SPMV)
@@ -317,7 +237,7 @@ __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT
     int stage = 0;
     XT acc[kDiagR] = {};
     while (cur.c < a.c1) {
-        const Group nxt = stage_next(stage ^ 1);
+        const DiagGroup nxt = stage_next(stage ^ 1);
         const int row = cur.c * kDiagRows + lane;
         const VT* st = ring + stage * (kDiagU * kDiagRows);
         if (cur.left & 1) group_fma<true, VT, XT>(a.x + row, st, cur, lane, acc);
@@ -359,11 +279,6 @@ __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT
             *a.counter = 0u;
         }
     }
-}
-
-template <typename VT>
-constexpr int diag_smem() {
-    return (kDiagNT / 32) * kDiagStages * kDiagU * kDiagRows * (int)sizeof(VT);
 }
 
 template <int MODE, typename VT, typename XT>

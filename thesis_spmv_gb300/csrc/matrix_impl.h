@@ -63,9 +63,10 @@ struct pwmgpu_matrix {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     bool loaded = false;
-    // No load-time launch tuning (the serving loop's matrices: its batched
-    // kernels do not use the handle's launch variant).
-    bool skip_tune = false;
+    // A serving loop's matrix: no load-time launch tuning (the batched kernels
+    // do not use the handle's launch variant), and no merge-path plan where
+    // the matrix fits diagonal slices.
+    bool batched = false;
 
     DevMatrix M;
 
@@ -252,6 +253,8 @@ int build_plan(pwmgpu_matrix* m);
 int ensure_vectors(pwmgpu_matrix* m);
 int ensure_fvectors(pwmgpu_matrix* m);
 int ensure_low_values(pwmgpu_matrix* m, bool allow_bf16, int* cfg, const void** valp, int* pgrid);
+// The diagonal slices' FP32 values, or BF16 ones where allowed and exact (*cfg).
+int diag_low(pwmgpu_matrix* m, bool allow_bf16, int* cfg);
 bool low_precision_floor(double rel, double prev_rel);
 bool sell_for(pwmgpu_matrix* m, int cfg);
 

@@ -272,6 +272,15 @@ int build_col16(pwmgpu_matrix* m) {
 
 // The merge-path plan (and, with run_tuner, the load-time launch tuner).
 int build_merge(pwmgpu_matrix* m, bool run_tuner) {
+    // diagonal slices where the matrix fits them (no memory: the merge plan alone)
+    const bool diag =
+        diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count, m->stream) == 0;
+    if (diag && m->batched) {
+        dfree(m->M.col);
+        dfree(m->M.val);
+        m->loaded = true;
+        return PWMGPU_OK;
+    }
     const long long total = (long long)m->M.nor + m->M.nnz;
     const MergeGeom g = merge_geometry(m->cfg);
     m->tm = g.wm;
@@ -295,10 +304,6 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
     TRY(build_col16(m));
     // fix-up descriptors; without them (no memory) the search-based fix-up runs
     (void)build_fix_runs(m->P, m->M.row_start, m->M.nor, m->sm_count, m->stream);
-    // diagonal slices where the matrix fits them (no memory: the merge plan
-    // alone); the serving loop's batched kernels do not read them
-    if (!m->skip_tune)
-        (void)diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count, m->stream);
     dfree(m->M.col);
     dfree(m->M.val);
     m->l1 = m->P.colp16 ? 2 : 0;
@@ -331,7 +336,7 @@ int build_plan(pwmgpu_matrix* m) {
         TRY(build_format(m));
         return tune_csb(m);
     }
-    return build_merge(m, !m->skip_tune);
+    return build_merge(m, !m->batched);
 }
 }  // namespace pwmgpu
 namespace {
@@ -584,7 +589,10 @@ int ensure_bf16_exact(pwmgpu_matrix* m) {
     int* flag = reinterpret_cast<int*>(m->barrier + 2);
     int h = 0;
     CU(cudaMemsetAsync(flag, 0, sizeof(int), m->stream));
-    CU(launch_bf16_exact(m->P.valp, mli_storage_elems(m->M.nnz, m->P.nsub), flag, m->sm_count, m->stream));
+    if (m->diag.nslices)  // (absent elements are stored as 0)
+        CU(launch_bf16_exact(m->diag.val64, m->diag.elems, flag, m->sm_count, m->stream));
+    else
+        CU(launch_bf16_exact(m->P.valp, mli_storage_elems(m->M.nnz, m->P.nsub), flag, m->sm_count, m->stream));
     CU(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     CU(cudaStreamSynchronize(m->stream));
     m->bf16_exact = h == 0 ? 1 : 0;
@@ -628,6 +636,17 @@ bool diag_for(pwmgpu_matrix* m, int cfg) {
     if (cfg == kCfgF64) return true;
     return m->low_format == PWMGPU_LOWFMT_AUTO &&
            diag_low_values(m->diag, cfg == kCfgBF16, m->sm_count, m->stream) == 0;
+}
+
+int diag_low(pwmgpu_matrix* m, bool allow_bf16, int* cfg) {
+    *cfg = kCfgF32;
+    if (allow_bf16) {
+        TRY(ensure_bf16_exact(m));
+        if (m->bf16_exact == 1) *cfg = kCfgBF16;
+    }
+    if (diag_low_values(m->diag, *cfg == kCfgBF16, m->sm_count, m->stream) != 0)
+        return fail(PWMGPU_ERR_NOMEM, "no memory for the low-precision values");
+    return PWMGPU_OK;
 }
 
 // The SELL-32 copy with values of configuration cfg (FP32 or BF16), built on

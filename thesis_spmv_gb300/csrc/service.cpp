@@ -32,10 +32,27 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
-// Precision classes; the FP32 / BF16 iterations of matrices that fit the
-// SELL-32 layout run in their own classes (kernel per layout).
-enum { kClsF64 = 0, kClsF32 = 1, kClsBF16 = 2, kClsF32Sell = 3, kClsBF16Sell = 4, kNumCls = 5 };
-constexpr int kSides = kNumCls - 1;  // forked streams of a round (the F64 class runs on the service stream)
+// Classes by precision and layout (a kernel for each): merge path, SELL-32
+// for the FP32 / BF16 iterations of banded matrices, diagonal slices for
+// stencils in every precision.
+enum {
+    kClsF64 = 0,
+    kClsF32 = 1,
+    kClsBF16 = 2,
+    kClsF32Sell = 3,
+    kClsBF16Sell = 4,
+    kClsF64Diag = 5,
+    kClsF32Diag = 6,
+    kClsBF16Diag = 7,
+    kNumCls = 8
+};
+struct ClsKind {
+    int cfg, layout;
+};
+constexpr ClsKind kCls[kNumCls] = {{kCfgF64, kBatchMerge}, {kCfgF32, kBatchMerge}, {kCfgBF16, kBatchMerge},
+                                   {kCfgF32, kBatchSell},  {kCfgBF16, kBatchSell}, {kCfgF64, kBatchDiag},
+                                   {kCfgF32, kBatchDiag},  {kCfgBF16, kBatchDiag}};
+constexpr int kSides = kNumCls - 1;  // forked streams of a round (its first class runs on the service stream)
 
 // Residual at which a mixed solve leaves the FP32 / BF16 phase (as in
 // pwmgpu_solve).
@@ -147,8 +164,11 @@ struct pwmsvc {
     std::vector<void*> deferred;  // device frees of the matrix builds, made after the round
     ClassDev cls[kNumCls];
     bool dirty = true;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
+    // One captured round per set of classes with live solves (bit c: class c),
+    // made when the set first occurs: a class without solves costs a round
+    // nothing (its kernels did little, but each was a full grid in the graph).
+    unsigned mask = 0;
+    std::map<unsigned, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;
     int64_t submitted = 0, finished = 0, failed = 0, rounds = 0;
     double gpu_ms = 0.0;
 
@@ -158,8 +178,10 @@ struct pwmsvc {
         free_deferred(deferred);
         for (auto& kv : all)
             if (kv.second->m) pwmgpu_destroy(kv.second->m);
-        if (gexec) cudaGraphExecDestroy(gexec);
-        if (graph) cudaGraphDestroy(graph);
+        for (auto& g : graphs) {
+            cudaGraphExecDestroy(g.second.second);
+            cudaGraphDestroy(g.second.first);
+        }
         for (auto& c : cls) {
             dfree(c.dT);
             dfree(c.d_slots);
@@ -191,8 +213,15 @@ int prepare_low(Req* r) {
     pwmgpu_matrix* m = r->m;
     const pwmsvc_request& q = r->spec;
     int cfg = kCfgF32, pg = 0;
-    TRY(ensure_low_values(m, q.precision == PWMGPU_PREC_MIXED, &cfg, &r->valp_low, &pg));
     TRY(ensure_fvectors(m));
+    if (m->diag.nslices) {
+        TRY(diag_low(m, q.precision == PWMGPU_PREC_MIXED, &cfg));
+        r->valp_low = cfg == kCfgBF16 ? m->diag.valbf : (const void*)m->diag.val32;
+        r->low_cls = cfg == kCfgBF16 ? kClsBF16Diag : kClsF32Diag;
+        CU(cudaStreamSynchronize(m->stream));
+        return PWMGPU_OK;
+    }
+    TRY(ensure_low_values(m, q.precision == PWMGPU_PREC_MIXED, &cfg, &r->valp_low, &pg));
     if (sell_for(m, cfg)) {
         r->valp_low = cfg == kCfgBF16 ? m->sell.valbf : (const void*)m->sell.val32;
         r->low_cls = cfg == kCfgBF16 ? kClsBF16Sell : kClsF32Sell;
@@ -208,7 +237,7 @@ int admit(pwmsvc* S, Req* r) {
     const pwmsvc_request& q = r->spec;
     TRY(pwmgpu_create(PWMGPU_FMT_MERGE, 1, &r->m));
     pwmgpu_matrix* m = r->m;
-    m->skip_tune = true;
+    m->batched = true;
     if (q.source == PWMSVC_SRC_POISSON) {
         TRY(pwmgpu_generate_poisson(m, q.grid_m, q.grid_n));
     } else if (q.source == PWMSVC_SRC_RANDOM) {
@@ -239,7 +268,7 @@ int admit(pwmsvc* S, Req* r) {
     } else {
         CU(launch_fill_uniform(m->dx, r->n, q.x0_seed, m->sm_count, m->stream));
     }
-    r->cls = kClsF64;
+    r->cls = m->diag.nslices ? kClsF64Diag : kClsF64;
     r->low = false;
     // MIXED: the probe round first, the low-precision copies only if the
     // solve takes the low phase
@@ -261,7 +290,9 @@ int reset_state(pwmsvc* S, int slot) {
 }
 
 int rebuild_tables(pwmsvc* S) {
+    S->mask = 0;
     for (int c = 0; c < kNumCls; ++c) {
+        const bool sell = kCls[c].layout == kBatchSell, diag = kCls[c].layout == kBatchDiag;
         ClassDev& D = S->cls[c];
         std::vector<BatchSlot> hs;
         int tiles = 0, fix = 0, rows = 0;
@@ -271,7 +302,7 @@ int rebuild_tables(pwmsvc* S) {
             BatchSlot b{};
             b.row_start = m->M.row_start;
             b.colp = m->P.colp;
-            b.valp = r->low ? r->valp_low : (const void*)m->P.valp;
+            b.valp = r->low ? r->valp_low : diag ? (const void*)m->diag.val64 : (const void*)m->P.valp;
             b.rec = m->P.rec;
             b.masks = m->P.masks;
             b.subc = m->P.subc;
@@ -280,16 +311,21 @@ int rebuild_tables(pwmsvc* S) {
             b.carries = m->carries;
             b.nor = m->M.nor;
             b.nsub = m->P.nsub;
-            if (c == kClsF32Sell || c == kClsBF16Sell) {  // slices instead of sub-tiles, no fix-up
+            if (sell) {  // slices instead of sub-tiles, no fix-up
                 b.soff = m->sell.soff;
                 b.col16 = m->sell.col16;
                 b.nsub = m->sell.nslices;
+            } else if (diag) {
+                b.drec = m->diag.rec;
+                b.doffs = m->diag.offs;
+                b.dmasks = static_cast<const unsigned*>(m->diag.masks);
+                b.nsub = m->diag.nslices;
             }
             b.tile0 = tiles;
-            b.nfix = (c == kClsF32Sell || c == kClsBF16Sell) ? (b.nsub + kSellGroup - 1) / kSellGroup
-                                                              : (b.nsub + kFixTiles - 1) / kFixTiles;
+            b.nfix = diag ? 0 : sell ? (b.nsub + kSellGroup - 1) / kSellGroup : (b.nsub + kFixTiles - 1) / kFixTiles;
             b.fix0 = fix;
-            b.nrow = (b.nor + kRowChunk - 1) / kRowChunk;
+            b.rchunk = row_chunk(b.nor);
+            b.nrow = (b.nor + b.rchunk - 1) / b.rchunk;
             b.row0 = rows;
             b.state = r->slot;
             tiles += b.nsub;
@@ -297,6 +333,8 @@ int rebuild_tables(pwmsvc* S) {
             rows += b.nrow;
             hs.push_back(b);
         }
+        if (hs.empty()) continue;  // not in the round
+        S->mask |= 1u << c;
         if (D.slots_cap < hs.size() || !D.d_slots) {
             dfree(D.d_slots);
             D.slots_cap = 0;
@@ -312,10 +350,8 @@ int rebuild_tables(pwmsvc* S) {
         }
         TRY(grow(&D.row_part, &D.row_cap, 2 * (size_t)rows + 2));
         TRY(grow(&D.res_part, &D.res_cap, (size_t)rows + 1));
-        if (c == kClsF32Sell || c == kClsBF16Sell) TRY(grow(&D.grp_part, &D.grp_cap, (size_t)fix + 1));
-        if (!hs.empty())
-            CU(cudaMemcpyAsync(D.d_slots, hs.data(), hs.size() * sizeof(BatchSlot), cudaMemcpyHostToDevice,
-                               S->stream));
+        if (sell) TRY(grow(&D.grp_part, &D.grp_cap, (size_t)fix + 1));
+        CU(cudaMemcpyAsync(D.d_slots, hs.data(), hs.size() * sizeof(BatchSlot), cudaMemcpyHostToDevice, S->stream));
         BatchTable T{};
         T.nslots = (int)hs.size();
         T.ntiles = tiles;
@@ -337,17 +373,25 @@ int rebuild_tables(pwmsvc* S) {
     return PWMGPU_OK;
 }
 
-// The round: three class branches forked from S->stream.
+// The round: a branch per class with live solves, forked from S->stream (the
+// first of them runs on it).
 int enqueue_round(pwmsvc* S) {
     const int C = S->cfg.round_iterations;
+    int side = 0, first = -1;
     CU(cudaEventRecord(S->fork_ev, S->stream));
-    for (int i = 0; i < kSides; ++i) CU(cudaStreamWaitEvent(S->side[i], S->fork_ev, 0));
-    CU(launch_batch_round(kCfgF64, S->cls[kClsF64].dT, C, S->sm_count, S->stream));
-    CU(launch_batch_round(kCfgF32, S->cls[kClsF32].dT, C, S->sm_count, S->side[0]));
-    CU(launch_batch_round(kCfgBF16, S->cls[kClsBF16].dT, C, S->sm_count, S->side[1]));
-    CU(launch_batch_round(kCfgF32, S->cls[kClsF32Sell].dT, C, S->sm_count, S->side[2], true));
-    CU(launch_batch_round(kCfgBF16, S->cls[kClsBF16Sell].dT, C, S->sm_count, S->side[3], true));
-    for (int i = 0; i < kSides; ++i) {
+    for (int c = 0; c < kNumCls; ++c) {
+        if (!(S->mask >> c & 1u)) continue;
+        if (first < 0) {
+            first = c;
+            continue;
+        }
+        CU(cudaStreamWaitEvent(S->side[side], S->fork_ev, 0));
+        CU(launch_batch_round(kCls[c].cfg, S->cls[c].dT, C, S->sm_count, S->side[side], kCls[c].layout));
+        ++side;
+    }
+    if (first >= 0)
+        CU(launch_batch_round(kCls[first].cfg, S->cls[first].dT, C, S->sm_count, S->stream, kCls[first].layout));
+    for (int i = 0; i < side; ++i) {
         CU(cudaEventRecord(S->join_ev[i], S->side[i]));
         CU(cudaStreamWaitEvent(S->stream, S->join_ev[i], 0));
     }
@@ -355,22 +399,31 @@ int enqueue_round(pwmsvc* S) {
 }
 
 int run_round(pwmsvc* S) {
-    if (S->cfg.use_graph && !S->gexec) {
-        CU(cudaStreamBeginCapture(S->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = enqueue_round(S);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(S->stream, &g);
-        if (rc != PWMGPU_OK) {
-            if (g) cudaGraphDestroy(g);
-            return rc;
+    cudaGraphExec_t exec = nullptr;
+    if (S->cfg.use_graph) {
+        auto it = S->graphs.find(S->mask);
+        if (it == S->graphs.end()) {
+            CU(cudaStreamBeginCapture(S->stream, cudaStreamCaptureModeThreadLocal));
+            int rc = enqueue_round(S);
+            cudaGraph_t g = nullptr;
+            cudaError_t e = cudaStreamEndCapture(S->stream, &g);
+            if (rc != PWMGPU_OK || e != cudaSuccess) {
+                if (g) cudaGraphDestroy(g);
+                return rc != PWMGPU_OK ? rc : fail(PWMGPU_ERR_CUDA, "round capture: %s", cudaGetErrorString(e));
+            }
+            cudaGraphExec_t x = nullptr;
+            e = cudaGraphInstantiate(&x, g, 0);
+            if (e != cudaSuccess) {
+                cudaGraphDestroy(g);
+                return fail(PWMGPU_ERR_CUDA, "round graph: %s", cudaGetErrorString(e));
+            }
+            it = S->graphs.emplace(S->mask, std::make_pair(g, x)).first;
         }
-        if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "round capture: %s", cudaGetErrorString(e));
-        S->graph = g;
-        CU(cudaGraphInstantiate(&S->gexec, S->graph, 0));
+        exec = it->second.second;
     }
     CU(cudaEventRecord(S->ev0, S->stream));
-    if (S->gexec) {
-        CU(cudaGraphLaunch(S->gexec, S->stream));
+    if (exec) {
+        CU(cudaGraphLaunch(exec, S->stream));
     } else {
         TRY(enqueue_round(S));
     }
@@ -480,7 +533,7 @@ int after_round(pwmsvc* S, int* finished) {
                 TRY(reset_state(S, r->slot));
                 r->exact_set = false;
                 r->low = false;
-                r->cls = kClsF64;
+                r->cls = m->diag.nslices ? kClsF64Diag : kClsF64;
                 r->rounds_in_phase = 0;
                 S->dirty = true;
             }
@@ -648,8 +701,10 @@ int pwmsvc_step(pwmsvc* s, int32_t* live, int32_t* queued, int32_t* finished) {
             }
         }
         TRY(run_round(s));
-        CU(cudaMemcpyAsync(s->h_states, s->d_states, sizeof(SlotState) * (size_t)s->cfg.max_live,
-                           cudaMemcpyDeviceToHost, s->stream));
+        int used = 0;  // states in use lie below it
+        for (const Req* r : s->live) used = std::max(used, r->slot + 1);
+        CU(cudaMemcpyAsync(s->h_states, s->d_states, sizeof(SlotState) * (size_t)used, cudaMemcpyDeviceToHost,
+                           s->stream));
         CU(cudaMemcpyAsync(s->h_status, s->d_status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     }
     // admission: FIFO while slots and the HBM budget allow (by the requests'
