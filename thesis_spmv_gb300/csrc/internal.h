@@ -257,14 +257,25 @@ cudaError_t launch_random_fill(const uint64_t* thr, int max_len, int n, uint64_t
 long long scan_scratch_elems(long long n);
 cudaError_t launch_inclusive_scan(int32_t* a, long long n, int32_t* scratch, cudaStream_t st);
 
-// triplet.cu: triplet -> CRS on the device (stable LSD radix sort by (row, col))
+// triplet.cu: triplet -> CRS on the device (rows bucketed and sorted in shared
+// memory, or a stable LSD radix sort by (row, col))
 struct TripletScan {
     unsigned long long bad;   // first entry with a row or column out of range (~0 when none)
     unsigned int unsorted_rc; // input not sorted by (row, col)
     unsigned int unsorted_c;  // input not sorted by column
+    int longest;              // entries of the longest row
+    int pad;
 };
 cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long long nnz, int32_t nor, int32_t noc,
-                                int32_t* cnt, TripletScan* flags, int sm_count, cudaStream_t st);
+                                int32_t* cnt, int32_t* pos, TripletScan* flags, int sm_count, cudaStream_t st);
+// Rows of at most `longest` entries can be sorted by launch_triplet_rows: CRS
+// from the row starts and the scan's arrival numbers pos (which receive the
+// sorted rows with rows_out); rec: triplet_rec_bytes of scratch.
+bool triplet_rows_fit(int longest);
+size_t triplet_rec_bytes(long long nnz);
+cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
+                                long long nnz, const int32_t* row_start, int32_t nor, void* rec, int32_t* col,
+                                double* val, bool rows_out, int sm_count, cudaStream_t st);
 long long triplet_sort_table_elems(long long nnz);
 int triplet_sort_passes(int32_t nor, int32_t noc, bool col_passes);
 cudaError_t launch_triplet_sort(const int32_t* rows, const int32_t* cols, long long nnz, int32_t nor, int32_t noc,

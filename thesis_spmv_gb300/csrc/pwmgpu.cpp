@@ -1301,21 +1301,23 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
                       const int32_t* cols, const double* vals, int32_t* h_rows, int32_t* h_cols, double* h_vals) {
     int32_t* cnt = nullptr;
     int32_t* scan_scratch = nullptr;
+    int32_t* pos = nullptr;
+    unsigned char* rec = nullptr;
     TripletScan* dflags = nullptr;
     unsigned long long *keys_a = nullptr, *keys_b = nullptr;
-    int32_t *src_a = nullptr, *src_b = nullptr, *tab = nullptr;
+    int32_t *src_a = nullptr, *src_b = nullptr, *tab = nullptr, *tab_scratch = nullptr;
     bool matrix_touched = false;
     int rc = PWMGPU_OK;
     do {
-        const long long tab_elems = triplet_sort_table_elems(nnz);
-        const long long scan_n = std::max<long long>(nor, tab_elems);
         if ((rc = dalloc(&cnt, (size_t)nor + 1)) != PWMGPU_OK) break;
-        if ((rc = dalloc(&scan_scratch, (size_t)scan_scratch_elems(scan_n))) != PWMGPU_OK) break;
+        if ((rc = dalloc(&scan_scratch, (size_t)scan_scratch_elems(nor))) != PWMGPU_OK) break;
+        if ((rc = dalloc(&pos, (size_t)nnz)) != PWMGPU_OK) break;
         if ((rc = dalloc(&dflags, 1)) != PWMGPU_OK) break;
-        TripletScan flags{~0ull, 0u, 0u};
+        TripletScan flags{~0ull, 0u, 0u, 0, 0};
         cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nor + 1), m->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dflags, &flags, sizeof flags, cudaMemcpyHostToDevice, m->stream);
-        if (e == cudaSuccess) e = launch_triplet_scan(rows, cols, nnz, nor, noc, cnt, dflags, m->sm_count, m->stream);
+        if (e == cudaSuccess)
+            e = launch_triplet_scan(rows, cols, nnz, nor, noc, cnt, pos, dflags, m->sm_count, m->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, dflags, sizeof flags, cudaMemcpyDeviceToHost, m->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "triplet scan: %s", cudaGetErrorString(e)); break; }
@@ -1337,28 +1339,39 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
         if ((rc = alloc_matrix(m, nor, noc, nnz)) != PWMGPU_OK) break;
         e = cudaMemcpyAsync(m->M.row_start, cnt, sizeof(int32_t) * ((size_t)nor + 1), cudaMemcpyDeviceToDevice,
                             m->stream);
+        int32_t* sorted_rows = nullptr;
         if (e == cudaSuccess && nnz > 0 && !flags.unsorted_rc) {
             // already in CRS order: the columns and values are the input
             e = cudaMemcpyAsync(m->M.col, cols, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToDevice, m->stream);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(m->M.val, vals, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice,
                                     m->stream);
+        } else if (e == cudaSuccess && nnz > 0 && triplet_rows_fit(flags.longest)) {
+            if ((rc = dalloc(&rec, triplet_rec_bytes(nnz))) != PWMGPU_OK) break;
+            e = launch_triplet_rows(rows, cols, vals, pos, nnz, m->M.row_start, nor, rec, m->M.col, m->M.val,
+                                    h_rows != nullptr, m->sm_count, m->stream);
+            sorted_rows = pos;
         } else if (e == cudaSuccess && nnz > 0) {
+            const long long tab_elems = triplet_sort_table_elems(nnz);
+            dfree(pos);
             if ((rc = dalloc(&keys_a, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&keys_b, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&src_a, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&src_b, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&tab, (size_t)tab_elems)) != PWMGPU_OK) break;
+            if ((rc = dalloc(&tab_scratch, (size_t)scan_scratch_elems(tab_elems))) != PWMGPU_OK) break;
             unsigned long long* keys = nullptr;
-            int32_t* src = nullptr;
             e = launch_triplet_sort(rows, cols, nnz, nor, noc, flags.unsorted_c != 0, keys_a, src_a, keys_b, src_b,
-                                    tab, scan_scratch, &keys, &src, m->sm_count, m->stream);
+                                    tab, tab_scratch, &keys, &sorted_rows, m->sm_count, m->stream);
             // the sorted rows (for the caller's triplet) overwrite the source indices
             if (e == cudaSuccess)
-                e = launch_triplet_gather(keys, src, vals, nnz, m->M.col, m->M.val, h_rows ? src : nullptr,
-                                          m->sm_count, m->stream);
+                e = launch_triplet_gather(keys, sorted_rows, vals, nnz, m->M.col, m->M.val,
+                                          h_rows ? sorted_rows : nullptr, m->sm_count, m->stream);
+        }
+        if (sorted_rows) {
             if (e == cudaSuccess && h_rows)
-                e = cudaMemcpyAsync(h_rows, src, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToHost, m->stream);
+                e = cudaMemcpyAsync(h_rows, sorted_rows, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToHost,
+                                    m->stream);
             if (e == cudaSuccess && h_cols)
                 e = cudaMemcpyAsync(h_cols, m->M.col, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToHost,
                                     m->stream);
@@ -1371,12 +1384,15 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
     } while (0);
     dfree(cnt);
     dfree(scan_scratch);
+    dfree(pos);
+    dfree(rec);
     dfree(dflags);
     dfree(keys_a);
     dfree(keys_b);
     dfree(src_a);
     dfree(src_b);
     dfree(tab);
+    dfree(tab_scratch);
     if (rc != PWMGPU_OK) {
         if (matrix_touched) m->release_matrix();
         return rc;
