@@ -348,7 +348,7 @@ int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const 
     unsigned char* tmp = nullptr;
     int rc = 2;
     do {
-        if (cudaMalloc((void**)&tmp, scan_at + sizeof(int32_t) * (size_t)scan_scratch_elems(ns)) != cudaSuccess) break;
+        if (dev_alloc((void**)&tmp, scan_at + sizeof(int32_t) * (size_t)scan_scratch_elems(ns)) != cudaSuccess) break;
         Head* dh = reinterpret_cast<Head*>(tmp);
         int32_t* ptr = reinterpret_cast<int32_t*>(tmp + ptr_at);
         if (cudaMemsetAsync(tmp, 0, ptr_at + sizeof(int32_t), st) != cudaSuccess) break;
@@ -369,7 +369,7 @@ int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const 
                      mb = up(sizeof(SlotMask) * (slots + 1)), ob = up(sizeof(int32_t) * (slots + 1)),
                      nb = sizeof(double) * kDiagMaxCtas * (size_t)sm_count;
         if (launch_inclusive_scan(ptr + 1, ns, reinterpret_cast<int32_t*>(tmp + scan_at), st) != cudaSuccess) break;
-        if (cudaMalloc(&D.mem, vb + rb + mb + ob + nb) != cudaSuccess) {
+        if (dev_alloc(&D.mem, vb + rb + mb + ob + nb) != cudaSuccess) {
             D.mem = nullptr;
             break;
         }
@@ -386,6 +386,7 @@ int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const 
         D.elems = (long long)elems;
         rc = 0;
     } while (0);
+    (void)cudaStreamSynchronize(st);
     dev_free(tmp);
     if (rc) {
         (void)cudaGetLastError();
@@ -397,7 +398,7 @@ int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const 
 int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st) {
     void** dst = bf16 ? &D.valbf : (void**)&D.val32;
     if (*dst) return 0;
-    if (cudaMalloc(dst, (bf16 ? sizeof(__nv_bfloat16) : sizeof(float)) * ((size_t)D.elems + 8)) != cudaSuccess) {
+    if (dev_alloc(dst, (bf16 ? sizeof(__nv_bfloat16) : sizeof(float)) * ((size_t)D.elems + 8)) != cudaSuccess) {
         (void)cudaGetLastError();
         *dst = nullptr;
         return 2;

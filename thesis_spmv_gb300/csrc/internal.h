@@ -45,15 +45,16 @@ struct MergeGeom {
 
 // Per-matrix plan of the merge-path kernel: sub-tile boundaries, metadata,
 // row-end masks and the lane-interleaved column / FP64 value arrays.
-// Device frees.  cudaFree waits for all work on the device, so a build that
-// runs beside other kernels (the serving loop builds admitted matrices while
-// its round runs) would wait for them at every free.  defer_frees(&list)
-// makes this thread's dev_free calls append to `list` instead, until
-// defer_frees(nullptr); free_deferred(list) then frees them (after the caller
-// has synchronised the work that used them).
+// devmem.cpp: device blocks from the device's pool.  A block is ready on every
+// stream when dev_alloc returns; dev_free waits for nothing, so the work that
+// used the block has been synchronised before.
+cudaError_t dev_alloc(void** out, size_t bytes);
 void dev_free(void* p);
-void defer_frees(std::vector<void*>* list);
-void free_deferred(std::vector<void*>& list);
+// Bytes the current device's pool holds without using them.
+size_t dev_idle_bytes();
+// A pinned host block of 128 bytes.
+cudaError_t pinned_alloc(void** out);
+void pinned_free(void* p);
 
 struct MliPlan {
     int nsub = 0;

@@ -36,10 +36,10 @@ template <typename T>
 inline int dalloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+    cudaError_t e = dev_alloc((void**)p, count * sizeof(T));
     if (e != cudaSuccess) {
         *p = nullptr;
-        return fail(PWMGPU_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
+        return fail(PWMGPU_ERR_NOMEM, "device allocation of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
     }
     return PWMGPU_OK;
 }
@@ -159,6 +159,10 @@ struct pwmgpu_matrix {
         cudaEvent_t ev_start = nullptr;
     } pipe;
 
+    // Buffers replaced by larger ones while work on the stream (or a graph
+    // captured from it) may still use them.
+    std::vector<void*> outgrown;
+
     // host-facing vector buffers
     double* dx = nullptr;
     double* dy = nullptr;
@@ -184,7 +188,11 @@ struct pwmgpu_matrix {
         pwmgpu::dfree(coh.units);
         coh = decltype(coh)();
     }
+    // (the buffers go back without a wait: the handle's work ends first)
     void release_matrix() {
+        cudaStreamSynchronize(stream);
+        for (void* p : outgrown) pwmgpu::dev_free(p);
+        outgrown.clear();
         pwmgpu::dfree(M.row_start);
         pwmgpu::dfree(M.col);
         pwmgpu::dfree(M.val);
@@ -233,7 +241,7 @@ struct pwmgpu_matrix {
         pwmgpu::dfree(small);
         pwmgpu::dfree(status);
         pwmgpu::dfree(barrier);
-        if (hres) cudaFreeHost(hres);
+        pwmgpu::pinned_free(hres);
         hres = nullptr;
         pwmgpu::dfree(dx);
         pwmgpu::dfree(dy);

@@ -1347,9 +1347,9 @@ int build_fix_runs(MliPlan& P, const int32_t* row_start, int nor, int sm_count, 
     int rc = 0;
     const int nb = (P.nsub + 255) / 256;
     do {
-        if (cudaMalloc((void**)&desc, sizeof(int4) * (size_t)P.nsub) != cudaSuccess ||
-            cudaMalloc((void**)&scan_scratch, sizeof(int) * (size_t)scan_scratch_elems(P.nsub + 1)) != cudaSuccess ||
-            cudaMalloc((void**)&P.run_pre, sizeof(int) * ((size_t)P.nsub + 1)) != cudaSuccess) {
+        if (dev_alloc((void**)&desc, sizeof(int4) * (size_t)P.nsub) != cudaSuccess ||
+            dev_alloc((void**)&scan_scratch, sizeof(int) * (size_t)scan_scratch_elems(P.nsub + 1)) != cudaSuccess ||
+            dev_alloc((void**)&P.run_pre, sizeof(int) * ((size_t)P.nsub + 1)) != cudaSuccess) {
             rc = 1;
             break;
         }
@@ -1365,16 +1365,17 @@ int build_fix_runs(MliPlan& P, const int32_t* row_start, int nor, int sm_count, 
             break;
         }
         P.nruns = total;
-        if (cudaMalloc((void**)&P.runs, sizeof(int4) * (size_t)(total > 0 ? total : 1)) != cudaSuccess) { rc = 1; break; }
+        if (dev_alloc((void**)&P.runs, sizeof(int4) * (size_t)(total > 0 ? total : 1)) != cudaSuccess) { rc = 1; break; }
         if (total > 0) k_run_compact<<<nb, 256, 0, st>>>(P.run_pre, desc, P.nsub, P.runs);
         if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = 1;
     } while (0);
-    if (desc) dev_free(desc);
-    if (scan_scratch) dev_free(scan_scratch);
+    (void)cudaStreamSynchronize(st);
+    dev_free(desc);
+    dev_free(scan_scratch);
     if (rc) {
         (void)cudaGetLastError();
-        if (P.runs) dev_free(P.runs);
-        if (P.run_pre) dev_free(P.run_pre);
+        dev_free(P.runs);
+        dev_free(P.run_pre);
         P.runs = nullptr;
         P.run_pre = nullptr;
         P.nruns = 0;

@@ -42,34 +42,23 @@ int fail(int code, const char* fmt, ...) {
 
 namespace {
 
-int ensure_cap(double** p, size_t* cap, size_t need) {
+// Room for `need` elements in one of the handle's buffers.  The buffer it
+// replaces may still be in use on the stream: it goes back with the matrix
+// (twice the room each time bounds what waits there).
+template <typename T>
+int ensure_cap(pwmgpu_matrix* m, T** p, size_t* cap, size_t need) {
     if (*cap >= need && *p) return PWMGPU_OK;
-    dfree(*p);
-    *cap = 0;
-    TRY(dalloc(p, need));
-    *cap = need;
+    const size_t want = std::max(need, 2 * *cap);
+    T* q = nullptr;
+    TRY(dalloc(&q, want));
+    if (*p) m->outgrown.push_back(*p);
+    *p = q;
+    *cap = want;
     return PWMGPU_OK;
 }
 
 }  // namespace
 namespace pwmgpu {
-namespace {
-thread_local std::vector<void*>* g_deferred_frees = nullptr;
-}
-
-void dev_free(void* p) {
-    if (!p) return;
-    if (g_deferred_frees) g_deferred_frees->push_back(p);
-    else cudaFree(p);
-}
-
-void defer_frees(std::vector<void*>* list) { g_deferred_frees = list; }
-
-void free_deferred(std::vector<void*>& list) {
-    for (void* p : list) cudaFree(p);
-    list.clear();
-}
-
 int check_status(pwmgpu_matrix* m) {
     int st = 0;
     CU(cudaMemcpyAsync(&st, m->status, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
@@ -168,7 +157,7 @@ int build_format(pwmgpu_matrix* m) {
             CU(cudaMemcpyAsync(c.units, units.data(), sizeof(int) * units.size(), cudaMemcpyHostToDevice, m->stream));
     }
     CU(cudaStreamSynchronize(m->stream));
-    TRY(ensure_cap(&m->partials, &m->partials_cap, (size_t)2 * dot_grid(m->M.nor, m->sm_count) + 64));
+    TRY(ensure_cap(m, &m->partials, &m->partials_cap, (size_t)2 * dot_grid(m->M.nor, m->sm_count) + 64));
     m->loaded = true;
     return PWMGPU_OK;
 }
@@ -254,7 +243,7 @@ int build_col16(pwmgpu_matrix* m) {
     }
     if (rc == PWMGPU_OK && e == cudaSuccess && !wide) {
         const size_t elems = (size_t)mli_storage_elems(m->M.nnz, P.nsub);
-        if (cudaMalloc((void**)&P.colp16, elems * sizeof(uint16_t)) != cudaSuccess) {
+        if (dev_alloc((void**)&P.colp16, elems * sizeof(uint16_t)) != cudaSuccess) {
             (void)cudaGetLastError();
             P.colp16 = nullptr;
         } else {
@@ -263,6 +252,7 @@ int build_col16(pwmgpu_matrix* m) {
             if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         }
     }
+    (void)cudaStreamSynchronize(m->stream);
     dfree(cbase);
     dfree(flag);
     if (rc != PWMGPU_OK) return rc;
@@ -313,12 +303,12 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
     m->pgrid32 = power_persistent_grid(kCfgF32, m->num_tiles, m->sm_count, m->l1);
     m->pgridbf = power_persistent_grid(kCfgBF16, m->num_tiles, m->sm_count, m->l1);
     const int pmax = std::max(m->pgrid, std::max(m->pgrid32, m->pgridbf));
-    TRY(ensure_cap(&m->carries, &m->carries_cap, (size_t)m->num_tiles + 1));
-    TRY(ensure_cap(&m->partials, &m->partials_cap,
+    TRY(ensure_cap(m, &m->carries, &m->carries_cap, (size_t)m->num_tiles + 1));
+    TRY(ensure_cap(m, &m->partials, &m->partials_cap,
                    (size_t)std::max(std::max(m->grid, 2 * pmax), 2 * dot_grid(m->M.nor, m->sm_count)) + 64));
     // shares of a power step's ||y||^2: at most one per SpMV CTA (16 resident
     // CTAs per SM at most, 4 warps per CTA) and one per fix-up CTA
-    TRY(ensure_cap(&m->npart, &m->npart_cap,
+    TRY(ensure_cap(m, &m->npart, &m->npart_cap,
                    (size_t)power_norm_parts(m->P, (int)std::min<long long>(((long long)m->num_tiles + 3) / 4,
                                                                            16LL * m->sm_count)) + 64));
     CU(cudaStreamSynchronize(m->stream));
@@ -346,27 +336,20 @@ namespace pwmgpu {
 int ensure_vectors(pwmgpu_matrix* m) {
     size_t need = (size_t)std::max(m->M.nor, m->M.noc) + kPad;
     if (m->vec_cap >= need) return PWMGPU_OK;
-    dfree(m->dx);
-    dfree(m->dy);
-    m->vec_cap = 0;
-    TRY(dalloc(&m->dx, need));
-    TRY(dalloc(&m->dy, need));
-    m->vec_cap = need;
+    size_t cx = m->vec_cap, cy = m->vec_cap;
+    TRY(ensure_cap(m, &m->dx, &cx, need));
+    TRY(ensure_cap(m, &m->dy, &cy, need));
+    m->vec_cap = std::min(cx, cy);
     return PWMGPU_OK;
 }
 }  // namespace pwmgpu
 namespace {
 
-int ensure_nsq(pwmgpu_matrix* m, size_t need) { return ensure_cap(&m->nsq, &m->nsq_cap, need + 1); }
+int ensure_nsq(pwmgpu_matrix* m, size_t need) { return ensure_cap(m, &m->nsq, &m->nsq_cap, need + 1); }
 
 // Magnitude keys of `need` iterates, zeroed (the steps atomicMax into them).
 int ensure_mxk(pwmgpu_matrix* m, size_t need) {
-    if (m->mxk_cap < need || !m->mxk) {
-        dfree(m->mxk);
-        m->mxk_cap = 0;
-        TRY(dalloc(&m->mxk, need));
-        m->mxk_cap = need;
-    }
+    TRY(ensure_cap(m, &m->mxk, &m->mxk_cap, need));
     CU(cudaMemsetAsync(m->mxk, 0, sizeof(unsigned int) * need, m->stream));
     return PWMGPU_OK;
 }
@@ -606,7 +589,7 @@ int ensure_low_values(pwmgpu_matrix* m, bool allow_bf16, int* cfg, const void** 
         TRY(ensure_bf16_exact(m));
         if (m->bf16_exact == 1) {
             if (!m->valbf) {
-                CU(cudaMalloc(&m->valbf, 2 * (size_t)elems + 16));
+                CU(dev_alloc(&m->valbf, 2 * (size_t)elems + 16));
                 CU(cudaMemsetAsync(m->valbf, 0, 2 * (size_t)elems + 16, m->stream));
                 CU(launch_mli_convert(m->P, kCfgBF16, m->valbf, m->sm_count, m->stream));
             }
@@ -688,12 +671,10 @@ namespace pwmgpu {
 int ensure_fvectors(pwmgpu_matrix* m) {
     size_t need = (size_t)std::max(m->M.nor, m->M.noc) + kPad;
     if (m->fvec_cap >= need) return PWMGPU_OK;
-    dfree(m->fx);
-    dfree(m->fy);
-    m->fvec_cap = 0;
-    TRY(dalloc(&m->fx, need));
-    TRY(dalloc(&m->fy, need));
-    m->fvec_cap = need;
+    size_t cx = m->fvec_cap, cy = m->fvec_cap;
+    TRY(ensure_cap(m, &m->fx, &cx, need));
+    TRY(ensure_cap(m, &m->fy, &cy, need));
+    m->fvec_cap = std::min(cx, cy);
     return PWMGPU_OK;
 }
 }  // namespace pwmgpu
@@ -976,7 +957,8 @@ int plan_pipeline(pwmgpu_matrix* m) {
                          : launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p.rec.data(), d, sizeof(int) * (diag ? 1 : 4) * K, cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+    const cudaError_t se = cudaStreamSynchronize(m->stream);
+    if (e == cudaSuccess) e = se;
     dfree(d);
     if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "pipeline plan: %s", cudaGetErrorString(e));
     // diagonal slices: a chunk is a range of slices, its rows its own
@@ -1143,7 +1125,7 @@ int pwmgpu_device_info(int* sm_count, size_t* free_bytes, size_t* total_bytes) {
     size_t f = 0, t = 0;
     CU(cudaMemGetInfo(&f, &t));
     if (sm_count) *sm_count = sms;
-    if (free_bytes) *free_bytes = f;
+    if (free_bytes) *free_bytes = f + dev_idle_bytes();
     if (total_bytes) *total_bytes = t;
     return PWMGPU_OK;
 }
@@ -1171,8 +1153,8 @@ int pwmgpu_create(int format, int partitions, pwmgpu_matrix** out) {
         if ((rc = dalloc(&m->status, 4)) != PWMGPU_OK) break;
         if ((rc = dalloc(&m->small, 16)) != PWMGPU_OK) break;
         if ((rc = dalloc(&m->barrier, 4)) != PWMGPU_OK) break;
-        e = cudaMallocHost((void**)&m->hres, 16 * sizeof(double));
-        if (e != cudaSuccess) { m->hres = nullptr; rc = fail(PWMGPU_ERR_NOMEM, "cudaMallocHost: %s", cudaGetErrorString(e)); break; }
+        e = pinned_alloc((void**)&m->hres);
+        if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_NOMEM, "pinned memory: %s", cudaGetErrorString(e)); break; }
         cudaMemsetAsync(m->counter, 0, 4 * sizeof(unsigned int), m->stream);
         cudaMemsetAsync(m->status, 0, 4 * sizeof(int), m->stream);
         e = cudaStreamSynchronize(m->stream);
@@ -1267,6 +1249,7 @@ int pwmgpu_generate_random(pwmgpu_matrix* m, int32_t n, uint64_t seed, int lengt
         if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "random generator: %s", cudaGetErrorString(e)); break; }
     } while (0);
+    (void)cudaStreamSynchronize(m->stream);
     dfree(dthr);
     dfree(dtotal);
     dfree(scratch);
@@ -1284,7 +1267,8 @@ struct TripletIn {
     int32_t* rows = nullptr;
     int32_t* cols = nullptr;
     double* vals = nullptr;
-    void release() {
+    void release(cudaStream_t st) {
+        (void)cudaStreamSynchronize(st);
         dfree(rows);
         dfree(cols);
         dfree(vals);
@@ -1353,7 +1337,6 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
             sorted_rows = pos;
         } else if (e == cudaSuccess && nnz > 0) {
             const long long tab_elems = triplet_sort_table_elems(nnz);
-            dfree(pos);
             if ((rc = dalloc(&keys_a, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&keys_b, (size_t)nnz)) != PWMGPU_OK) break;
             if ((rc = dalloc(&src_a, (size_t)nnz)) != PWMGPU_OK) break;
@@ -1382,6 +1365,7 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
         if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "triplet to CRS: %s", cudaGetErrorString(e)); break; }
     } while (0);
+    (void)cudaStreamSynchronize(m->stream);
     dfree(cnt);
     dfree(scan_scratch);
     dfree(pos);
@@ -1449,7 +1433,7 @@ int pwmgpu_load_triplets(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "triplet upload: %s", cudaGetErrorString(e)); break; }
         rc = load_triplets_dev(m, nor, noc, nnz, in.rows, in.cols, in.vals, rows, cols, vals);
     } while (0);
-    in.release();
+    in.release(m->stream);
     return rc;
 }
 
@@ -1504,6 +1488,7 @@ int pwmgpu_stats(pwmgpu_matrix* m, pwmgpu_matrix_stats* out) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         if (e != cudaSuccess) rc = fail(PWMGPU_ERR_CUDA, "matrix statistics: %s", cudaGetErrorString(e));
     } while (0);
+    (void)cudaStreamSynchronize(m->stream);
     dfree(blocks);
     dfree(brow);
     dfree(rp);
@@ -1555,7 +1540,8 @@ int pwmgpu_get_csr(pwmgpu_matrix* m, int32_t* row_start, int32_t* col_ind, doubl
             e = cudaMemcpyAsync(col_ind, dc, sizeof(int32_t) * (size_t)m->M.nnz, cudaMemcpyDeviceToHost, m->stream);
         if (rc == PWMGPU_OK && e == cudaSuccess)
             e = cudaMemcpyAsync(vals, dv, sizeof(double) * (size_t)m->M.nnz, cudaMemcpyDeviceToHost, m->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+        const cudaError_t se = cudaStreamSynchronize(m->stream);
+        if (e == cudaSuccess) e = se;
         dfree(dc);
         dfree(dv);
         if (rc != PWMGPU_OK) return rc;
@@ -1626,7 +1612,8 @@ int pwmgpu_merge_partition(pwmgpu_matrix* m, int32_t parts, int32_t* coords) {
     cudaError_t e = launch_merge_partition(m->M.row_start, m->M.nor, m->M.nnz, ipt, parts, d, m->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(coords, d, sizeof(int2) * ((size_t)parts + 1), cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+    const cudaError_t se = cudaStreamSynchronize(m->stream);
+    if (e == cudaSuccess) e = se;
     dev_free(d);
     if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "merge partition: %s", cudaGetErrorString(e));
     return PWMGPU_OK;
@@ -1755,7 +1742,7 @@ int pwmgpu_load_triplets_rows(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "triplet upload: %s", cudaGetErrorString(e)); break; }
         rc = load_triplets_dev(m, last_row - first_row, noc, bn, in.rows, in.cols, in.vals, nullptr, nullptr, nullptr);
     } while (0);
-    in.release();
+    in.release(m->stream);
     return rc;
 }
 

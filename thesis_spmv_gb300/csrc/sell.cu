@@ -216,8 +216,8 @@ int sell_build(SellPlan& S, const int32_t* row_start, const int32_t* col, const 
     int rc = 0;
     do {
         if (S.state == 0) {
-            if (cudaMalloc((void**)&S.soff, sizeof(int32_t) * ((size_t)ns + 1)) != cudaSuccess ||
-                cudaMalloc((void**)&total, sizeof(unsigned long long)) != cudaSuccess) {
+            if (dev_alloc((void**)&S.soff, sizeof(int32_t) * ((size_t)ns + 1)) != cudaSuccess ||
+                dev_alloc((void**)&total, sizeof(unsigned long long)) != cudaSuccess) {
                 rc = 2;
                 break;
             }
@@ -238,11 +238,11 @@ int sell_build(SellPlan& S, const int32_t* row_start, const int32_t* col, const 
                 rc = 1;
                 break;
             }
-            if (cudaMalloc((void**)&scratch, sizeof(int32_t) * (size_t)scan_scratch_elems(ns)) != cudaSuccess ||
+            if (dev_alloc((void**)&scratch, sizeof(int32_t) * (size_t)scan_scratch_elems(ns)) != cudaSuccess ||
                 launch_inclusive_scan(S.soff + 1, ns, scratch, st) != cudaSuccess ||
-                cudaMalloc((void**)&S.col16, sizeof(uint16_t) * ((size_t)h + 16)) != cudaSuccess ||
-                cudaMalloc((void**)&S.npart, sizeof(double) * (8 * (size_t)sm_count + 64)) != cudaSuccess ||
-                cudaMalloc((void**)&flag, sizeof(int)) != cudaSuccess || cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) {
+                dev_alloc((void**)&S.col16, sizeof(uint16_t) * ((size_t)h + 16)) != cudaSuccess ||
+                dev_alloc((void**)&S.npart, sizeof(double) * (8 * (size_t)sm_count + 64)) != cudaSuccess ||
+                dev_alloc((void**)&flag, sizeof(int)) != cudaSuccess || cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) {
                 rc = 2;
                 break;
             }
@@ -252,11 +252,11 @@ int sell_build(SellPlan& S, const int32_t* row_start, const int32_t* col, const 
         void** dst = bf16 ? &S.valbf : (void**)&S.val32;
         if (*dst == nullptr) {
             const size_t esz = bf16 ? sizeof(__nv_bfloat16) : sizeof(float);
-            if (cudaMalloc(dst, esz * ((size_t)S.stored + 16)) != cudaSuccess) {
+            if (dev_alloc(dst, esz * ((size_t)S.stored + 16)) != cudaSuccess) {
                 rc = 2;
                 break;
             }
-            if (!flag && (cudaMalloc((void**)&flag, sizeof(int)) != cudaSuccess ||
+            if (!flag && (dev_alloc((void**)&flag, sizeof(int)) != cudaSuccess ||
                           cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess)) {
                 rc = 2;
                 break;
@@ -281,9 +281,10 @@ int sell_build(SellPlan& S, const int32_t* row_start, const int32_t* col, const 
         }
         S.state = 1;
     } while (0);
-    if (flag) dev_free(flag);
-    if (scratch) dev_free(scratch);
-    if (total) dev_free(total);
+    (void)cudaStreamSynchronize(st);
+    dev_free(flag);
+    dev_free(scratch);
+    dev_free(total);
     if (rc) {
         (void)cudaGetLastError();
         S.release();

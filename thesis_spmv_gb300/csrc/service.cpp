@@ -76,9 +76,9 @@ constexpr int kProbeRounds = 5;
 // there is no round to overlap, and the solves started later would only
 // finish later.
 constexpr int kAdmitPerStep = 32;
-// Host threads that build a step's admissions while its round runs (each on
-// its own stream: the builds are chains of short kernels, allocations and
-// stream syncs, bound by their latency, not by the GPU).
+// Host threads that build a step's admissions (each on its own stream: the
+// builds are chains of short kernels and stream syncs, bound by their latency,
+// not by the GPU).
 constexpr int kAdmitThreads = 8;
 
 struct Req {
@@ -161,7 +161,6 @@ struct pwmsvc {
     std::vector<int> free_states;
     int* d_status = nullptr;
     int* h_status = nullptr;  // pinned: read back while the host admits requests
-    std::vector<void*> deferred;  // device frees of the matrix builds, made after the round
     ClassDev cls[kNumCls];
     bool dirty = true;
     // One captured round per set of classes with live solves (bit c: class c),
@@ -175,7 +174,6 @@ struct pwmsvc {
     double now() const { return std::chrono::duration<double>(Clock::now() - t0).count(); }
 
     void release() {
-        free_deferred(deferred);
         for (auto& kv : all)
             if (kv.second->m) pwmgpu_destroy(kv.second->m);
         for (auto& g : graphs) {
@@ -581,7 +579,7 @@ int pwmsvc_create(const pwmsvc_config* cfg, pwmsvc** out) {
             size_t f = 0, t = 0;
             e = cudaMemGetInfo(&f, &t);
             if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "cudaMemGetInfo: %s", cudaGetErrorString(e)); break; }
-            S->cfg.hbm_budget_bytes = (size_t)(0.9 * (double)f);
+            S->cfg.hbm_budget_bytes = (size_t)(0.9 * (double)(f + dev_idle_bytes()));
         }
         if ((rc = dalloc(&S->d_states, (size_t)c.max_live)) != PWMGPU_OK) break;
         if ((rc = dalloc(&S->d_status, 4)) != PWMGPU_OK) break;
@@ -708,9 +706,7 @@ int pwmsvc_step(pwmsvc* s, int32_t* live, int32_t* queued, int32_t* finished) {
         CU(cudaMemcpyAsync(s->h_status, s->d_status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     }
     // admission: FIFO while slots and the HBM budget allow (by the requests'
-    // estimates), the builds on up to kAdmitThreads host threads; their
-    // device frees wait until the round is done (a cudaFree now would wait
-    // for the round)
+    // estimates), the builds on up to kAdmitThreads host threads
     std::vector<Req*> batch;
     size_t planned = s->in_use;
     const int cap = ran ? kAdmitPerStep : s->cfg.max_live;
@@ -726,32 +722,24 @@ int pwmsvc_step(pwmsvc* s, int32_t* live, int32_t* queued, int32_t* finished) {
         batch.push_back(r);
     }
     std::vector<int> built(batch.size(), PWMGPU_OK);
-    // several builders only beside a round: with the device idle (a batch
-    // submitted at once) one thread built the 256-matrix batch faster (178
-    // vs 170 solves/s; its 128 small random matrices 870 vs 760)
-    const int nt = ran ? (int)std::min<size_t>((size_t)kAdmitThreads, batch.size()) : 1;
+    // (32 requests with the device idle: 7.2 ms on one thread, 4.4 on eight)
+    const int nt = (int)std::min<size_t>((size_t)kAdmitThreads, batch.size());
     if (nt <= 1) {
-        defer_frees(&s->deferred);
         for (size_t i = 0; i < batch.size(); ++i) built[i] = admit(s, batch[i]);
-        defer_frees(nullptr);
     } else {
-        std::vector<std::vector<void*>> frees((size_t)nt + 1);
         std::atomic<int> next{0};
-        auto work = [&](size_t slot) {
+        auto work = [&]() {
             cudaSetDevice(s->device);
-            defer_frees(&frees[slot]);
             for (int i; (i = next.fetch_add(1)) < (int)batch.size();) built[(size_t)i] = admit(s, batch[(size_t)i]);
-            defer_frees(nullptr);
         };
         std::vector<std::thread> th;
         try {
-            for (int t = 0; t < nt; ++t) th.emplace_back(work, (size_t)t);
+            for (int t = 1; t < nt; ++t) th.emplace_back(work);
         } catch (const std::system_error&) {
             // no more threads: the ones started and this one share the rest
         }
-        work((size_t)nt);
+        work();
         for (auto& t : th) t.join();
-        for (auto& f : frees) s->deferred.insert(s->deferred.end(), f.begin(), f.end());
     }
     std::vector<Req*> admitted;
     for (size_t i = 0; i < batch.size(); ++i) {
@@ -776,7 +764,6 @@ int pwmsvc_step(pwmsvc* s, int32_t* live, int32_t* queued, int32_t* finished) {
     }
     if (ran) {
         const cudaError_t se = cudaStreamSynchronize(s->stream);
-        free_deferred(s->deferred);
         CU(se);
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, s->ev0, s->ev1) == cudaSuccess) s->gpu_ms += ms;
@@ -792,7 +779,6 @@ int pwmsvc_step(pwmsvc* s, int32_t* live, int32_t* queued, int32_t* finished) {
     }
     for (Req* r : admitted) s->live.push_back(r);
     if (!admitted.empty()) s->dirty = true;
-    free_deferred(s->deferred);
     if (live) *live = (int32_t)s->live.size();
     if (queued) *queued = (int32_t)s->queue.size();
     if (finished) *finished = fin;
