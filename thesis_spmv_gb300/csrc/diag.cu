@@ -418,7 +418,7 @@ cudaError_t launch_diag_maxcol(const DiagPlan& D, int nor, int noc, int K, int* 
 }
 
 cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, int noc, const void* x, void* y,
-                             const DiagStep& s, int sm_count, cudaStream_t st) {
+                             const SliceStep& s, int sm_count, cudaStream_t st) {
     const int c1 = s.c1 < 0 ? D.nslices : s.c1;
     double* np = s.nsq_out ? D.npart : nullptr;
     if (cfg == kCfgF64)

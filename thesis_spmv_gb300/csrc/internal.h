@@ -127,7 +127,7 @@ int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st);
 // kModePower: y = 2^e A x and *nsq_out = ||y||^2 (when given; counter zero
 // between launches); kModeScale: y = 2^e A x and atomicMax(*mx_out) of y's
 // magnitude keys.  e from *mx_in, else *nsq_in, else 0.
-struct DiagStep {
+struct SliceStep {
     const unsigned int* mx_in = nullptr;
     const double* nsq_in = nullptr;
     unsigned int* mx_out = nullptr;
@@ -137,12 +137,40 @@ struct DiagStep {
     bool pdl = true;
 };
 cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, int noc, const void* x, void* y,
-                             const DiagStep& s, int sm_count, cudaStream_t st);
+                             const SliceStep& s, int sm_count, cudaStream_t st);
 // Pipelined host-array SpMV: out[p] = the largest column the slices of chunks
 // 0..p read (slices [0, nslices (p + 1) / K)).
 cudaError_t launch_diag_maxcol(const DiagPlan& D, int nor, int noc, int K, int* out, cudaStream_t st);
 int diag_slice_rows();
 void diag_warm_launch_caches();
+
+// rows.cu: rows sorted by length within windows of consecutive rows, in items
+// of 32, 8 or 1 rows (a warp each); no carries.
+struct RowsPlan {
+    int nitems = 0;              // 0: the matrix does not fit the layout
+    int windows = 0, wrows = 0;  // windows of wrows rows
+    int win[17] = {};            // first item of each window (then nitems)
+    long long elems = 0;         // stored elements (64 per unit)
+    void* mem = nullptr;         // the allocation that rec .. val64 and npart lie in
+    int4* rec = nullptr;         // per item: {first unit, units, first row in perm, log2 lanes per row << 8 | rows}
+    int32_t* perm = nullptr;     // the rows in item order
+    int32_t* col = nullptr;      // columns, -1: absent
+    double* val64 = nullptr;
+    float* val32 = nullptr;      // the same in FP32 (made on first use)
+    void* valbf = nullptr;       // the same in BF16 (made on first use)
+    double* npart = nullptr;     // per-CTA shares of ||y||^2
+    void release();
+};
+// 0 = built, 1 = the matrix does not fit, 2 = a CUDA error or no memory (R
+// stays empty).
+int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
+               bool narrow, int sm_count, cudaStream_t st);
+int rows_low_values(RowsPlan& R, bool bf16, int sm_count, cudaStream_t st);
+// Pipelined host-array SpMV: out[w] = the largest column of windows 0 .. w.
+cudaError_t launch_rows_maxcol(const RowsPlan& R, int* out, cudaStream_t st);
+// As launch_diag_spmv, over items [s.c0, s.c1).
+cudaError_t launch_rows_spmv(const RowsPlan& R, int cfg, int mode, const void* x, void* y, const SliceStep& s,
+                             cudaStream_t st);
 
 // l1: launch variant of the merge kernels.  Bit 0: 0 = most resident CTAs,
 // 1 = a smaller shared-memory carveout, more L1 for irregular gathers; bit 1:
@@ -277,6 +305,11 @@ size_t triplet_rec_bytes(long long nnz);
 cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
                                 long long nnz, const int32_t* row_start, int32_t nor, void* rec, int32_t* col,
                                 double* val, bool rows_out, int sm_count, cudaStream_t st);
+// One stable pass of the radix sort by the keys' byte at `shift` (tab:
+// triplet_sort_table_elems(n) words, scan_scratch for as many).
+cudaError_t launch_radix_pass(const unsigned long long* keys, const int32_t* src, long long n, int shift,
+                              int32_t* tab, int32_t* scan_scratch, unsigned long long* keys_out, int32_t* src_out,
+                              cudaStream_t st);
 long long triplet_sort_table_elems(long long nnz);
 int triplet_sort_passes(int32_t nor, int32_t noc, bool col_passes);
 cudaError_t launch_triplet_sort(const int32_t* rows, const int32_t* cols, long long nnz, int32_t nor, int32_t noc,

@@ -101,6 +101,7 @@ struct pwmgpu_matrix {
     int low_format = PWMGPU_LOWFMT_AUTO;
     // diagonal slices (nslices 0: the matrix does not fit them)
     pwmgpu::DiagPlan diag;
+    pwmgpu::RowsPlan rows;  // sorted row slices (nitems 0: not built)
 
     // scratch
     double* carries = nullptr;  // max(num_tiles, num_tiles32) doubles (also used as floats)
@@ -217,6 +218,7 @@ struct pwmgpu_matrix {
         bf16_exact = -1;
         sell.release();
         diag.release();
+        rows.release();
         M = DevMatrix();
         num_tiles = 0;
         loaded = false;

@@ -189,10 +189,10 @@ int tune(pwmgpu_matrix* m) {
     // variants: carveout (bit 0) x gathers through L1 or around it (bit 2)
     const int cand[4] = {0, 1, 4, 5};
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
-    // a matrix on diagonal slices runs the merge kernels only where the handle
+    // a matrix on slices runs the merge kernels only where the handle
     // asks for them: two timed runs do (36 -> 12 SpMVs, 1.4 ms of the load of
     // a 2048^2 stencil)
-    const int reps = m->diag.nslices ? 2 : 8;
+    const int reps = m->diag.nslices || m->rows.nitems ? 2 : 8;
     for (int c = 0; c < 4 && rc == PWMGPU_OK; ++c) {
         const int v = cand[c] | c16;
         const int grid = merge_grid(kCfgF64, m->num_tiles, m->sm_count, v);
@@ -249,7 +249,6 @@ int build_col16(pwmgpu_matrix* m) {
         } else {
             e = cudaMemsetAsync(P.colp16, 0, elems * sizeof(uint16_t), m->stream);
             if (e == cudaSuccess) e = launch_mli_col16(P, cbase, m->sm_count, m->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
         }
     }
     (void)cudaStreamSynchronize(m->stream);
@@ -290,8 +289,10 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
         CU(launch_merge_partition(m->M.row_start, m->M.nor, m->M.nnz, m->tm, P.nsub, P.subc, m->stream));
         CU(launch_mli_plan(m->M.row_start, m->M.col, m->M.val, P, m->sm_count, m->stream));
     }
-    CU(cudaStreamSynchronize(m->stream));
     TRY(build_col16(m));
+    if (!diag && !m->batched)
+        (void)rows_build(m->rows, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->P.colp16 != nullptr,
+                         m->sm_count, m->stream);
     // fix-up descriptors; without them (no memory) the search-based fix-up runs
     (void)build_fix_runs(m->P, m->M.row_start, m->M.nor, m->sm_count, m->stream);
     dfree(m->M.col);
@@ -418,11 +419,20 @@ int fp64_format(const pwmgpu_matrix* m) {
     return m->tuned_fmt > 0 ? m->tuned_fmt : PWMGPU_FMT_MERGE;
 }
 
+// A handle whose steps run on slices (diagonal ones, or sorted rows) rather
+// than the merge plan: one kernel per step, no fix-up.
+bool sliced(const pwmgpu_matrix* m) { return m->diag.nslices || m->rows.nitems; }
+
+cudaError_t launch_sliced(pwmgpu_matrix* m, int cfg, int mode, const void* x, void* y, const SliceStep& s) {
+    return m->diag.nslices ? launch_diag_spmv(m->diag, cfg, mode, m->M.nor, m->M.noc, x, y, s, m->sm_count, m->stream)
+                           : launch_rows_spmv(m->rows, cfg, mode, x, y, s, m->stream);
+}
+
 int spmv_f64(pwmgpu_matrix* m, const double* dx, double* dy) {
     if (fp64_format(m) != PWMGPU_FMT_MERGE) return spmv_format(m, fp64_format(m), dx, dy, nullptr);
     if (m->num_tiles == 0) return PWMGPU_OK;
-    if (m->diag.nslices) {
-        CU(launch_diag_spmv(m->diag, kCfgF64, kModeSpmv, m->M.nor, m->M.noc, dx, dy, DiagStep{}, m->sm_count, m->stream));
+    if (sliced(m)) {
+        CU(launch_sliced(m, kCfgF64, kModeSpmv, dx, dy, SliceStep{}));
         return PWMGPU_OK;
     }
     CU(launch_merge_spmv(kCfgF64, kModeSpmv, m->M, m->P.valp, m->P, m->grid, dx, dy, m->carries, nullptr, m->status,
@@ -447,13 +457,13 @@ bool norm_in_step(const pwmgpu_matrix* m, int grid) {
 // descriptors.
 int power_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double* nsq_in, double* nsq_out,
                    const unsigned int* mx_in = nullptr) {
-    if (m->diag.nslices) {
-        DiagStep s;
+    if (sliced(m)) {
+        SliceStep s;
         s.mx_in = mx_in;
         s.nsq_in = nsq_in;
         s.counter = m->counter + 2;
         s.nsq_out = nsq_out;
-        CU(launch_diag_spmv(m->diag, kCfgF64, kModePower, m->M.nor, m->M.noc, in, out, s, m->sm_count, m->stream));
+        CU(launch_sliced(m, kCfgF64, kModePower, in, out, s));
         return PWMGPU_OK;
     }
     if (norm_in_step(m, m->grid)) {
@@ -485,12 +495,12 @@ int power_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double
 // Needs the plan's run descriptors (norm_in_step).
 int scale_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double* nsq_in, const unsigned int* mx_in,
                    unsigned int* mx_out) {
-    if (m->diag.nslices) {
-        DiagStep s;
+    if (sliced(m)) {
+        SliceStep s;
         s.mx_in = mx_in;
         s.nsq_in = nsq_in;
         s.mx_out = mx_out;
-        CU(launch_diag_spmv(m->diag, kCfgF64, kModeScale, m->M.nor, m->M.noc, in, out, s, m->sm_count, m->stream));
+        CU(launch_sliced(m, kCfgF64, kModeScale, in, out, s));
         return PWMGPU_OK;
     }
     CU(launch_merge_spmv(kCfgF64, kModeScale, m->M, m->P.valp, m->P, m->grid, in, out, m->carries, nsq_in,
@@ -540,7 +550,7 @@ int power_device(pwmgpu_matrix* m, double* dx, double* dy, int32_t it) {
         // The last two steps compute the exact norms the final normalisation
         // uses; the steps before them only need the rescale exponent, from
         // their input's largest magnitude key (MODE_SCALE).
-        const bool scale = m->diag.nslices || norm_in_step(m, m->grid);
+        const bool scale = sliced(m) || norm_in_step(m, m->grid);
         if (scale) TRY(ensure_mxk(m, (size_t)it + 1));
         for (int k = 0; k < it; ++k) {
             const double* in = (k % 2 == 0) ? dx : dy;
@@ -610,15 +620,17 @@ int ensure_low_values(pwmgpu_matrix* m, bool allow_bf16, int* cfg, const void** 
     return PWMGPU_OK;
 }
 
-// Whether iterations of configuration cfg run on the diagonal slices: the
-// matrix fits them, and the handle asks for neither the persistent merge
+// Whether iterations of configuration cfg run on the handle's slices: the
+// matrix fits some, and the handle asks for neither the persistent merge
 // kernel nor (FP32 / BF16) the merge layout.  Makes the FP32 / BF16 values on
 // first use.
-bool diag_for(pwmgpu_matrix* m, int cfg) {
-    if (!m->diag.nslices || m->power_mode == PWMGPU_POWER_FUSED) return false;
+bool sliced_for(pwmgpu_matrix* m, int cfg) {
+    if (!sliced(m) || m->power_mode == PWMGPU_POWER_FUSED) return false;
     if (cfg == kCfgF64) return true;
-    return m->low_format == PWMGPU_LOWFMT_AUTO &&
-           diag_low_values(m->diag, cfg == kCfgBF16, m->sm_count, m->stream) == 0;
+    if (m->low_format != PWMGPU_LOWFMT_AUTO) return false;
+    const bool bf = cfg == kCfgBF16;
+    return (m->diag.nslices ? diag_low_values(m->diag, bf, m->sm_count, m->stream)
+                            : rows_low_values(m->rows, bf, m->sm_count, m->stream)) == 0;
 }
 
 int diag_low(pwmgpu_matrix* m, bool allow_bf16, int* cfg) {
@@ -693,8 +705,8 @@ struct ChunkOut {
 // differs.
 int solve_chunk(pwmgpu_matrix* m, int cfg, const void* valp, int pgrid, void* X, void* Y, int k0, int nk,
                 ChunkOut* o) {
-    if (diag_for(m, cfg)) {
-        // diagonal slices: one kernel per step; the steps before the last
+    if (sliced_for(m, cfg)) {
+        // slices: one kernel per step; the steps before the last
         // two track only the rescale's magnitude keys, the last one takes
         // the row pass for v_k . v_{k+1}
         const bool f32 = cfg != kCfgF64;
@@ -704,14 +716,13 @@ int solve_chunk(pwmgpu_matrix* m, int cfg, const void* valp, int pgrid, void* X,
             const void* in = (k & 1) ? Y : X;
             void* out = (k & 1) ? X : Y;
             const bool keys = k < k0 + nk - 2, last = k == k0 + nk - 1;
-            DiagStep s;
+            SliceStep s;
             if (k > k0 && k - 1 < k0 + nk - 2) s.mx_in = m->mxk + k;
             else if (k > 0) s.nsq_in = m->nsq + k;
             s.counter = m->counter + 2;
             if (keys) s.mx_out = m->mxk + k + 1;
             else if (!last) s.nsq_out = m->nsq + k + 1;
-            CU(launch_diag_spmv(m->diag, cfg, keys ? kModeScale : kModePower, m->M.nor, m->M.noc, in, out, s,
-                                m->sm_count, m->stream));
+            CU(launch_sliced(m, cfg, keys ? kModeScale : kModePower, in, out, s));
         }
         const int k = k0 + nk - 1;
         const void* in = (k & 1) ? Y : X;
@@ -860,8 +871,8 @@ int solve(pwmgpu_matrix* m, double* x, int32_t max_it, double tol, int precision
                 pg = m->pgridbf;
             }
         }
-        // (diagonal slices hold their own FP32 / BF16 values)
-        if (!diag_for(m, cfg)) TRY(ensure_low_values(m, precision == PWMGPU_PREC_MIXED, &cfg, &valp, &pg));
+        // (slices hold their own FP32 / BF16 values)
+        if (!sliced_for(m, cfg)) TRY(ensure_low_values(m, precision == PWMGPU_PREC_MIXED, &cfg, &valp, &pg));
         if (pg == 0 && m->power_mode == PWMGPU_POWER_FUSED)
             return fail(PWMGPU_ERR_UNSUPPORTED, "the fused power kernel cannot be made co-resident");
         TRY(ensure_fvectors(m));
@@ -949,24 +960,28 @@ int plan_pipeline(pwmgpu_matrix* m) {
     p.K = -1;
     const int K = kPipeChunks;
     if (m->num_tiles < 64 * K) return PWMGPU_OK;  // too small to gain from it
+    const bool rows = m->rows.nitems > 0;
+    if (rows && m->rows.windows != K) return PWMGPU_OK;
     int* d = nullptr;
     TRY(dalloc(&d, 4 * (size_t)K));
     p.rec.assign(4 * (size_t)K, 0);
     const bool diag = m->diag.nslices > 0;
     cudaError_t e = diag ? launch_diag_maxcol(m->diag, m->M.nor, m->M.noc, K, d, m->stream)
-                         : launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
+                    : rows ? launch_rows_maxcol(m->rows, d, m->stream)
+                           : launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(p.rec.data(), d, sizeof(int) * (diag ? 1 : 4) * K, cudaMemcpyDeviceToHost, m->stream);
+        e = cudaMemcpyAsync(p.rec.data(), d, sizeof(int) * (diag || rows ? 1 : 4) * K, cudaMemcpyDeviceToHost, m->stream);
     const cudaError_t se = cudaStreamSynchronize(m->stream);
     if (e == cudaSuccess) e = se;
     dfree(d);
     if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "pipeline plan: %s", cudaGetErrorString(e));
-    // diagonal slices: a chunk is a range of slices, its rows its own
-    if (diag)
+    // slices: a chunk is a range of diagonal slices or a window of sorted rows,
+    // its rows its own
+    if (diag || rows)
         for (int c = K - 1; c >= 0; --c) {
-            const int s0 = (int)((long long)m->diag.nslices * c / K);
+            const int s0 = diag ? (int)((long long)m->diag.nslices * c / K) : m->rows.win[c];
             const int mx = p.rec[(size_t)c];
-            const int rec[4] = {s0, s0 * diag_slice_rows(), 0, mx};
+            const int rec[4] = {s0, diag ? s0 * diag_slice_rows() : c * m->rows.wrows, 0, mx};
             std::copy(rec, rec + 4, p.rec.begin() + 4 * c);
         }
     // a run of sub-tiles may cross at most one chunk boundary: chunk first
@@ -975,7 +990,7 @@ int plan_pipeline(pwmgpu_matrix* m) {
         if (p.rec[4 * c + 1] <= p.rec[4 * (c - 1) + 1]) return PWMGPU_OK;
     for (int c = 1; c < K; ++c) p.rec[4 * c + 3] = std::max(p.rec[4 * c + 3], p.rec[4 * (c - 1) + 3]);
     p.fpre.assign(K + 1, 0);
-    if (m->P.runs && !diag) {
+    if (m->P.runs && !sliced(m)) {
         for (int c = 0; c < K; ++c)
             CU(cudaMemcpy(&p.fpre[(size_t)c], m->P.run_pre + p.rec[4 * c], sizeof(int), cudaMemcpyDeviceToHost));
         p.fpre[(size_t)K] = m->P.nruns;
@@ -1021,15 +1036,18 @@ bool sm_reachable_pageable(pwmgpu_matrix* m, const void* h) {
 int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
     auto& p = m->pipe;
     const int K = p.K, noc = m->M.noc, nor = m->M.nor;
-    const bool diag = m->diag.nslices > 0;
-    const int nsub = diag ? m->diag.nslices : m->num_tiles;
+    const bool own = sliced(m);  // a chunk's rows are its own
+    const int nsub = m->diag.nslices ? m->diag.nslices : m->rows.nitems ? m->rows.nitems : m->num_tiles;
     const bool x_sm = sm_reachable_pageable(m, x), y_sm = sm_reachable_pageable(m, y);
     // the streams start after earlier work on the handle's stream
     CU(cudaEventRecord(p.ev_start, m->stream));
     CU(cudaStreamWaitEvent(p.in, p.ev_start, 0));
     CU(cudaStreamWaitEvent(p.out, p.ev_start, 0));
-    for (int q = 0; q < kPipeX; ++q) {
-        const long long a = (long long)noc * q / kPipeX, b = (long long)noc * (q + 1) / kPipeX;
+    // (pieces of x and groups of chunks of at least 128 K rows: below that the
+    // launches cost more than the overlap gives)
+    const int nx = std::max(1, std::min(kPipeX, noc >> 17));
+    for (int q = 0; q < nx; ++q) {
+        const long long a = (long long)noc * q / nx, b = (long long)noc * (q + 1) / nx;
         if (b > a && x_sm)
             CU(launch_host_copy(x + a, m->dx + a, b - a, p.in));
         else if (b > a)
@@ -1038,7 +1056,7 @@ int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
     }
     auto piece_of = [&](int col) {  // the x piece holding column col
         int q = 0;
-        while (q + 1 < kPipeX && (long long)noc * (q + 1) / kPipeX <= col) ++q;
+        while (q + 1 < nx && (long long)noc * (q + 1) / nx <= col) ++q;
         return q;
     };
     auto chunk_tiles = [&](int c, int* t0, int* t1) {
@@ -1048,46 +1066,57 @@ int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
     // rows chunk c downloads: [lo_c, lo_{c+1})
     auto row_lo = [&](int c) { return c == 0 ? 0 : (c >= K ? nor : p.rec[4 * c + 1] + p.rec[4 * c + 2]); };
     int waited = -1;
-    for (int c = 0; c <= K; ++c) {
-        if (c < K) {
-            const int need = piece_of(p.rec[4 * c + 3]);
-            for (int q = waited + 1; q <= need; ++q) CU(cudaStreamWaitEvent(m->stream, p.ev_x[(size_t)q], 0));
-            waited = std::max(waited, need);
-            int t0, t1;
-            chunk_tiles(c, &t0, &t1);
-            if (diag) {
-                DiagStep s;
-                s.c0 = t0;
-                s.c1 = t1;
-                s.pdl = false;  // as launch_merge_spmv_range
-                CU(launch_diag_spmv(m->diag, kCfgF64, kModeSpmv, nor, noc, m->dx, m->dy, s, m->sm_count, m->stream));
-            } else {
-                const int grid = merge_grid(kCfgF64, t1 - t0, m->sm_count, m->l1);
-                CU(launch_merge_spmv_range(m->M, m->P, t0, t1, grid, m->dx, m->dy, m->carries, m->status, m->stream,
-                                           m->l1));
-            }
+    // the x pieces that chunks 0..c read have to be up
+    auto need_x = [&](int c) {
+        const int need = piece_of(p.rec[4 * c + 3]);
+        for (int q = waited + 1; q <= need; ++q) CU(cudaStreamWaitEvent(m->stream, p.ev_x[(size_t)q], 0));
+        waited = std::max(waited, need);
+        return PWMGPU_OK;
+    };
+    // the rows of chunks [f, f + n) go down
+    auto send_y = [&](int f, int n) {
+        CU(cudaEventRecord(p.ev_y[(size_t)f], m->stream));
+        CU(cudaStreamWaitEvent(p.out, p.ev_y[(size_t)f], 0));
+        const int r0 = row_lo(f), r1 = row_lo(f + n);
+        if (r1 > r0 && y_sm)
+            CU(launch_host_copy(m->dy + r0, y + r0, r1 - r0, p.out));
+        else if (r1 > r0)
+            CU(cudaMemcpyAsync(y + r0, m->dy + r0, sizeof(double) * (size_t)(r1 - r0), cudaMemcpyDeviceToHost, p.out));
+        return PWMGPU_OK;
+    };
+    if (own) {
+        // slices: a chunk's rows are its own, so they go down as soon as it is done
+        const int group = (int)std::min<long long>(K, ((long long)K * (1 << 17) + nor - 1) / nor);
+        for (int c = 0; c < K; c += group) {
+            const int n = std::min(group, K - c);
+            TRY(need_x(c + n - 1));
+            SliceStep s;
+            s.c0 = p.rec[4 * c];
+            s.c1 = c + n < K ? p.rec[4 * (c + n)] : nsub;
+            s.pdl = false;  // as launch_merge_spmv_range
+            CU(launch_sliced(m, kCfgF64, kModeSpmv, m->dx, m->dy, s));
+            TRY(send_y(c, n));
         }
-        // chunk f is done: its rows go down -- the chunk just launched (diagonal
-        // slices), or the one before it after the fix-up of its runs (they end
-        // by chunk c)
-        const int f = diag ? c : c - 1;
-        if (f >= 0 && f < K) {
-            int t0, t1;
-            chunk_tiles(f, &t0, &t1);
-            if (!diag && m->P.runs)
-                CU(launch_fix_runs_f64(kModeSpmv, m->P, p.fpre[(size_t)f], p.fpre[(size_t)f + 1], m->dy, m->carries,
+    }
+    for (int c = 0; !own && c <= K; ++c) {
+        int t0, t1;
+        if (c < K) {
+            TRY(need_x(c));
+            chunk_tiles(c, &t0, &t1);
+            const int grid = merge_grid(kCfgF64, t1 - t0, m->sm_count, m->l1);
+            CU(launch_merge_spmv_range(m->M, m->P, t0, t1, grid, m->dx, m->dy, m->carries, m->status, m->stream,
+                                       m->l1));
+        }
+        if (c >= 1) {
+            // chunk c-1: fix-up of its runs (they end by chunk c), then its rows go down
+            chunk_tiles(c - 1, &t0, &t1);
+            if (m->P.runs)
+                CU(launch_fix_runs_f64(kModeSpmv, m->P, p.fpre[(size_t)c - 1], p.fpre[(size_t)c], m->dy, m->carries,
                                        nullptr, m->stream));
-            else if (!diag)
+            else
                 CU(launch_merge_fixup_range(m->M, m->P.subc, nsub, t0, t1, m->dy, m->carries, m->stream,
                                             m->sm_count));
-            CU(cudaEventRecord(p.ev_y[(size_t)f], m->stream));
-            CU(cudaStreamWaitEvent(p.out, p.ev_y[(size_t)f], 0));
-            const int r0 = row_lo(f), r1 = row_lo(f + 1);
-            if (r1 > r0 && y_sm)
-                CU(launch_host_copy(m->dy + r0, y + r0, r1 - r0, p.out));
-            else if (r1 > r0)
-                CU(cudaMemcpyAsync(y + r0, m->dy + r0, sizeof(double) * (size_t)(r1 - r0), cudaMemcpyDeviceToHost,
-                                   p.out));
+            TRY(send_y(c - 1, 1));
         }
     }
     CU(cudaStreamSynchronize(p.out));
@@ -1633,9 +1662,8 @@ int pwmgpu_mv_device_f32(pwmgpu_matrix* m, const float* dx, float* dy) {
     if (m->format != PWMGPU_FMT_MERGE) return fail(PWMGPU_ERR_UNSUPPORTED, "FP32 SpMV runs on the merge format");
     if (m->M.nor > 0 && (!dx || !dy)) return fail(PWMGPU_ERR_INVALID, "null vector");
     if (m->num_tiles == 0) return PWMGPU_OK;
-    if (diag_for(m, kCfgF32)) {
-        CU(launch_diag_spmv(m->diag, kCfgF32, kModeSpmv, m->M.nor, m->M.noc, dx, dy, DiagStep{}, m->sm_count,
-                            m->stream));
+    if (sliced_for(m, kCfgF32)) {
+        CU(launch_sliced(m, kCfgF32, kModeSpmv, dx, dy, SliceStep{}));
         return PWMGPU_OK;
     }
     if (sell_for(m, kCfgF32)) {

@@ -352,7 +352,6 @@ cudaError_t launch_triplet_sort(const int32_t* rows, const int32_t* cols, long l
     *src_sorted = src_a;
     if (nnz <= 0) return cudaSuccess;
     k_trip_pack<<<stream_grid(nnz, sm_count), 256, 0, st>>>(rows, cols, nnz, keys_a, src_a);
-    const long long tiles = (nnz + kSortTile - 1) / kSortTile;
     int shifts[8], np = 0;
     if (col_passes)
         for (int s = 0; s < bits_for(noc); s += 8) shifts[np++] = s;
@@ -360,10 +359,8 @@ cudaError_t launch_triplet_sort(const int32_t* rows, const int32_t* cols, long l
     unsigned long long *ki = keys_a, *ko = keys_b;
     int32_t *si = src_a, *so = src_b;
     for (int p = 0; p < np; ++p) {
-        k_radix_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(ki, nnz, shifts[p], tab, (int)tiles);
-        cudaError_t e = launch_inclusive_scan(tab + 1, tiles * kRadixBins, scan_scratch, st);
+        const cudaError_t e = launch_radix_pass(ki, si, nnz, shifts[p], tab, scan_scratch, ko, so, st);
         if (e != cudaSuccess) return e;
-        k_radix_scatter<<<(unsigned)tiles, kSortThreads, 0, st>>>(ki, si, nnz, shifts[p], tab, (int)tiles, ko, so);
         unsigned long long* kt = ki;
         ki = ko;
         ko = kt;
@@ -373,6 +370,18 @@ cudaError_t launch_triplet_sort(const int32_t* rows, const int32_t* cols, long l
     }
     *keys_sorted = ki;
     *src_sorted = si;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_radix_pass(const unsigned long long* keys, const int32_t* src, long long n, int shift,
+                              int32_t* tab, int32_t* scan_scratch, unsigned long long* keys_out, int32_t* src_out,
+                              cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    const long long tiles = (n + kSortTile - 1) / kSortTile;
+    k_radix_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(keys, n, shift, tab, (int)tiles);
+    const cudaError_t e = launch_inclusive_scan(tab + 1, tiles * kRadixBins, scan_scratch, st);
+    if (e != cudaSuccess) return e;
+    k_radix_scatter<<<(unsigned)tiles, kSortThreads, 0, st>>>(keys, src, n, shift, tab, (int)tiles, keys_out, src_out);
     return cudaGetLastError();
 }
 
