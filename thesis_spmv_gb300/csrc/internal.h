@@ -299,11 +299,10 @@ cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long l
                                 int32_t* cnt, int32_t* pos, TripletScan* flags, int sm_count, cudaStream_t st);
 // Rows of at most `longest` entries can be sorted by launch_triplet_rows: CRS
 // from the row starts and the scan's arrival numbers pos (which receive the
-// sorted rows with rows_out); rec: triplet_rec_bytes of scratch.
+// sorted rows with rows_out); src: nnz words of scratch.
 bool triplet_rows_fit(int longest);
-size_t triplet_rec_bytes(long long nnz);
 cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
-                                long long nnz, const int32_t* row_start, int32_t nor, void* rec, int32_t* col,
+                                long long nnz, const int32_t* row_start, int32_t nor, int32_t* src, int32_t* col,
                                 double* val, bool rows_out, int sm_count, cudaStream_t st);
 // One stable pass of the radix sort by the keys' byte at `shift` (tab:
 // triplet_sort_table_elems(n) words, scan_scratch for as many).

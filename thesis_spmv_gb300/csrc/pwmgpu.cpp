@@ -1315,7 +1315,6 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
     int32_t* cnt = nullptr;
     int32_t* scan_scratch = nullptr;
     int32_t* pos = nullptr;
-    unsigned char* rec = nullptr;
     TripletScan* dflags = nullptr;
     unsigned long long *keys_a = nullptr, *keys_b = nullptr;
     int32_t *src_a = nullptr, *src_b = nullptr, *tab = nullptr, *tab_scratch = nullptr;
@@ -1360,8 +1359,8 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
                 e = cudaMemcpyAsync(m->M.val, vals, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice,
                                     m->stream);
         } else if (e == cudaSuccess && nnz > 0 && triplet_rows_fit(flags.longest)) {
-            if ((rc = dalloc(&rec, triplet_rec_bytes(nnz))) != PWMGPU_OK) break;
-            e = launch_triplet_rows(rows, cols, vals, pos, nnz, m->M.row_start, nor, rec, m->M.col, m->M.val,
+            if ((rc = dalloc(&src_a, (size_t)nnz)) != PWMGPU_OK) break;
+            e = launch_triplet_rows(rows, cols, vals, pos, nnz, m->M.row_start, nor, src_a, m->M.col, m->M.val,
                                     h_rows != nullptr, m->sm_count, m->stream);
             sorted_rows = pos;
         } else if (e == cudaSuccess && nnz > 0) {
@@ -1398,7 +1397,6 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
     dfree(cnt);
     dfree(scan_scratch);
     dfree(pos);
-    dfree(rec);
     dfree(dflags);
     dfree(keys_a);
     dfree(keys_b);

@@ -11,16 +11,20 @@
 //      returned), the longest row, and two order flags: "not sorted by (row,
 //      col)" and "not sorted by column".
 //   2. Already sorted by (row, col): col / val are the input, copied.
-//   3. Rows of at most kRowSortMax entries: k_trip_bucket writes each entry as
-//      a 16-byte record {column, index, value} to row_start + arrival number,
-//      then k_trip_rows sorts every row in shared memory by (column, index) --
-//      an element's place is the number of smaller keys in its row, so the
-//      order of the arrivals does not matter -- and writes col / val (and the
-//      sorted rows, for callers whose triplet is sorted in place, like the
-//      reference's).  Bound by the scattered 16-byte writes (a 32-byte sector
-//      each) and the row atomics; every other access is a stream.  21 M
-//      shuffled entries of a 2048^2 stencil: 3.4 ms of kernels with the radix
-//      sort, 1.35 ms so (scan 0.25, bucket 0.92, rows 0.18).
+//   3. Rows of at most kRowSortMax entries: k_trip_bucket writes each entry's
+//      index to row_start + arrival number, k_trip_rows sorts every row in
+//      shared memory by (column, index) -- an element's place is the number of
+//      smaller keys in its row, so the order of the arrivals does not matter
+//      -- and k_trip_vals gathers the values.  Bound by the row atomics, the
+//      scattered stores and the two gathers; every other access is a stream.
+//      Scattered stores of 4 bytes run at 196 G/s, of 16 bytes at 31 G/s (67
+//      and 268 MB), gathers at 260 G/s from what L2 holds and 117 G/s from 134
+//      MB: so the index alone is scattered, and columns and values are
+//      gathered one after the other.  Load of 21 M shuffled entries of a
+//      2048^2 stencil: 7.9 ms with the radix sort, 3.15 with scattered {column,
+//      index, value} records, 2.80 so (scan 0.24 ms, bucket 0.26, rows 0.26,
+//      values 0.27); sorted by column 2.40 -> 2.23 ms; 8 M entries of a random
+//      matrix 1.34 -> 1.20.
 //   4. Longer rows: a stable LSD radix sort of the packed key row << 32 | col
 //      with 8-bit digits: first the column digits (skipped when the input is
 //      already sorted by column -- a stable sort by a key that is already in
@@ -103,33 +107,25 @@ __global__ void k_trip_scan(const int32_t* __restrict__ rows, const int32_t* __r
 
 constexpr int kRowSortMax = 4096;  // entries of a row k_trip_rows sorts (32 KB of keys)
 constexpr int kRowSortRows = 512;  // rows per CTA
-constexpr int kRowSortNT = 256;
+// Threads per CTA: the keys of four CTAs leave L1 room for the gathers in
+// flight (256 threads, six CTAs: 0.54 ms on 21 M entries; so 0.26).
+constexpr int kRowSortNT = 512;
+constexpr int kTripU = 4;  // entries per thread whose loads go together
 
-struct __align__(16) TripRec {
-    int32_t col, src;
-    double val;
-};
-
-// rec[row_start[r] + arrival number] = the entry.  Four entries per thread
-// with their loads together: the row_start gathers hide behind each other.
-__global__ void __launch_bounds__(256) k_trip_bucket(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
-                                                     const double* __restrict__ vals,
-                                                     const int32_t* __restrict__ pos, long long nnz,
-                                                     const int32_t* __restrict__ row_start,
-                                                     TripRec* __restrict__ rec) {
-    constexpr int U = 4;
+// src[row_start[r] + arrival number] = the entry's index.  Four entries per
+// thread with their loads together: the row_start gathers hide behind each
+// other.
+__global__ void __launch_bounds__(256) k_trip_bucket(const int32_t* __restrict__ rows, const int32_t* __restrict__ pos,
+                                                     long long nnz, const int32_t* __restrict__ row_start,
+                                                     int32_t* __restrict__ src) {
+    constexpr int U = kTripU;
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long k0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; k0 < nnz; k0 += U * step) {
-        int32_t at[U], c[U];
-        double v[U];
+        int32_t at[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const long long k = k0 + u * step;
-            if (k < nnz) {
-                at[u] = __ldcs(rows + k);
-                c[u] = __ldcs(cols + k);
-                v[u] = __ldcs(vals + k);
-            }
+            if (k < nnz) at[u] = __ldcs(rows + k);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -139,17 +135,18 @@ __global__ void __launch_bounds__(256) k_trip_bucket(const int32_t* __restrict__
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const long long k = k0 + u * step;
-            if (k < nnz) rec[at[u]] = TripRec{c[u], (int32_t)k, v[u]};
+            if (k < nnz) src[at[u]] = (int32_t)k;
         }
     }
 }
 
 // Sort each row's records by (column, index).  A CTA takes kRowSortRows rows,
 // as many consecutive ones at a time as fit kRowSortMax keys.
-__global__ void __launch_bounds__(kRowSortNT) k_trip_rows(const TripRec* __restrict__ rec,
+__global__ void __launch_bounds__(kRowSortNT) k_trip_rows(int32_t* __restrict__ src,
+                                                          const int32_t* __restrict__ cols,
                                                           const int32_t* __restrict__ row_start, int32_t nor,
-                                                          int32_t* __restrict__ col, double* __restrict__ val,
-                                                          int32_t* __restrict__ rows_out) {
+                                                          int32_t* __restrict__ col, int32_t* __restrict__ rows_out) {
+    constexpr int U = kTripU;
     __shared__ unsigned long long key[kRowSortMax];
     __shared__ int start[kRowSortRows + 1];
     const int tid = threadIdx.x;
@@ -166,9 +163,19 @@ __global__ void __launch_bounds__(kRowSortNT) k_trip_rows(const TripRec* __restr
                 else hi = mid - 1;
             }
             const int base = start[a], m = start[b] - base;
-            for (int i = tid; i < m; i += kRowSortNT) {
-                const int2 q = __ldg(reinterpret_cast<const int2*>(rec + base + i));
-                key[i] = (unsigned long long)(uint32_t)q.x << 32 | (uint32_t)q.y;
+            for (int i0 = tid; i0 < m; i0 += U * kRowSortNT) {
+                uint32_t k[U];
+                int32_t c[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (i0 + u * kRowSortNT < m) k[u] = (uint32_t)__ldcs(src + base + i0 + u * kRowSortNT);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (i0 + u * kRowSortNT < m) c[u] = __ldg(cols + k[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (i0 + u * kRowSortNT < m)
+                        key[i0 + u * kRowSortNT] = (unsigned long long)(uint32_t)c[u] << 32 | k[u];
             }
             __syncthreads();
             for (int i = tid; i < m; i += kRowSortNT) {
@@ -182,13 +189,34 @@ __global__ void __launch_bounds__(kRowSortNT) k_trip_rows(const TripRec* __restr
                 const unsigned long long mine = key[i];
                 int at = s;
                 for (int j = s; j < t; ++j) at += key[j] < mine;
-                col[base + at] = (int32_t)(uint32_t)(mine >> 32);
-                val[base + at] = __ldg(&rec[base + i].val);
-                if (rows_out) rows_out[base + at] = (int32_t)(r0 + lo);
+                __stcs(col + base + at, (int32_t)(uint32_t)(mine >> 32));
+                __stcs(src + base + at, (int32_t)(uint32_t)mine);
+                if (rows_out) __stcs(rows_out + base + at, (int32_t)(r0 + lo));
             }
             __syncthreads();
             a = b;
         }
+    }
+}
+
+// val[i] = vals[src[i]].  After k_trip_rows and not in it: there the gathers
+// of the columns and of the values would evict each other from L2.
+__global__ void __launch_bounds__(256) k_trip_vals(const int32_t* __restrict__ src, const double* __restrict__ vals,
+                                                   long long nnz, double* __restrict__ val) {
+    constexpr int U = kTripU;
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long k0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; k0 < nnz; k0 += U * step) {
+        uint32_t at[U];
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * step < nnz) at[u] = (uint32_t)__ldcs(src + k0 + u * step);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * step < nnz) v[u] = __ldg(vals + at[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * step < nnz) __stcs(val + k0 + u * step, v[u]);
     }
 }
 
@@ -319,18 +347,17 @@ cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long l
 }
 
 bool triplet_rows_fit(int longest) { return longest <= kRowSortMax; }
-size_t triplet_rec_bytes(long long nnz) { return sizeof(TripRec) * (size_t)nnz; }
 
 cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
-                                long long nnz, const int32_t* row_start, int32_t nor, void* rec, int32_t* col,
+                                long long nnz, const int32_t* row_start, int32_t nor, int32_t* src, int32_t* col,
                                 double* val, bool rows_out, int sm_count, cudaStream_t st) {
     if (nnz <= 0) return cudaSuccess;
-    k_trip_bucket<<<stream_grid((nnz + 3) / 4, sm_count), 256, 0, st>>>(rows, cols, vals, pos, nnz, row_start,
-                                                                        static_cast<TripRec*>(rec));
+    k_trip_bucket<<<stream_grid((nnz + kTripU - 1) / kTripU, sm_count), 256, 0, st>>>(rows, pos, nnz, row_start, src);
     const long long ctas = ((long long)nor + kRowSortRows - 1) / kRowSortRows;
     // (the arrival numbers are done with: pos takes the sorted rows)
     k_trip_rows<<<(int)(ctas < 16LL * sm_count ? ctas : 16LL * sm_count), kRowSortNT, 0, st>>>(
-        static_cast<const TripRec*>(rec), row_start, nor, col, val, rows_out ? pos : nullptr);
+        src, cols, row_start, nor, col, rows_out ? pos : nullptr);
+    k_trip_vals<<<stream_grid((nnz + kTripU - 1) / kTripU, sm_count), 256, 0, st>>>(src, vals, nnz, val);
     return cudaGetLastError();
 }
 
