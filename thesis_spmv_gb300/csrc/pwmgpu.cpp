@@ -189,25 +189,29 @@ int tune(pwmgpu_matrix* m) {
     // variants: carveout (bit 0) x gathers through L1 or around it (bit 2)
     const int cand[4] = {0, 1, 4, 5};
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
-    // a matrix on slices runs the merge kernels only where the handle
-    // asks for them: two timed runs do (36 -> 12 SpMVs, 1.4 ms of the load of
-    // a 2048^2 stencil)
-    const int reps = m->diag.nslices || m->rows.nitems ? 2 : 8;
+    // A matrix on slices runs the merge kernels only where the handle asks for
+    // them: two timed runs over a quarter of the sub-tiles do (at least two
+    // waves of CTAs).  Load of a 2048^2 stencil: 2.67 ms with two runs over
+    // all of them, 2.18 so (the same variants chosen, stencils and irregular).
+    const bool side = m->diag.nslices || m->rows.nitems;
+    const int reps = side ? 2 : 8, tiles = side ? m->num_tiles / 4 : m->num_tiles;
     for (int c = 0; c < 4 && rc == PWMGPU_OK; ++c) {
         const int v = cand[c] | c16;
-        const int grid = merge_grid(kCfgF64, m->num_tiles, m->sm_count, v);
+        const int grid = merge_grid(kCfgF64, tiles, m->sm_count, v);
         cudaError_t e = cudaSuccess;
         for (int r = 0; r <= reps && e == cudaSuccess; ++r) {  // one warm-up, the rest timed
             if (r == 1) e = cudaEventRecord(e0, m->stream);
-            if (e == cudaSuccess)
-                e = launch_merge_spmv(kCfgF64, kModeSpmv, m->M, m->P.valp, m->P, grid, m->dx, m->dy, m->carries,
-                                      nullptr, m->status, m->stream, v);
+            if (e != cudaSuccess) continue;
+            e = side ? launch_merge_spmv_range(m->M, m->P, 0, tiles, grid, m->dx, m->dy, m->carries, m->status,
+                                               m->stream, v)
+                     : launch_merge_spmv(kCfgF64, kModeSpmv, m->M, m->P.valp, m->P, grid, m->dx, m->dy, m->carries,
+                                         nullptr, m->status, m->stream, v);
         }
         if (e == cudaSuccess) e = cudaEventRecord(e1, m->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[c], e0, e1);
         if (e != cudaSuccess) rc = fail(PWMGPU_ERR_CUDA, "launch tuning: %s", cudaGetErrorString(e));
-        ms[c] /= (float)reps;
+        ms[c] *= (float)m->num_tiles / ((float)reps * (float)tiles);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
