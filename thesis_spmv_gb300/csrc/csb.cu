@@ -14,7 +14,8 @@
 // the block row, every column window) and adds each element's product into
 // the y window, then writes its rows of y once.  Dense units (at least
 // kDenseUnit elements) stage their S-column x window in shared memory with a
-// TMA bulk copy (double-buffered, mbarriers) and are taken by the whole CTA;
+// TMA bulk copy (double-buffered, mbarriers; units in a row with the same
+// window share it) and are taken by the whole CTA;
 // a window's sparse units (a random matrix's blocks hold a few elements
 // each) are merged into one "flat" unit taken by the whole CTA, gathering x
 // through L1/L2 by global column -- staging 8 KB of x for a handful of
@@ -60,10 +61,14 @@ namespace {
 
 // Kernel variants (launch_csb_spmv's `variant`): bit 0 = 8 elements of a
 // dense unit per lane (else 4), bit 1 = 256 threads per CTA (else 128).
-// Every variant is launched with 1024 resident threads per SM (at most 64
-// registers; 24.6 KB of shared memory per CTA).  Variant 0 is the default;
-// the format autotuner times all four.
-constexpr int kCsbThreadsPerSM = 1024;
+// Resident CTAs per SM (24.6 KB of shared memory each): 7 of 128 threads, 4
+// of 256.  The loads in flight land in what shared memory leaves of L1, and
+// they bound a stencil: 4096^2 Poisson 227 us at 7 CTAs of 128
+// (about 4 % more at 6, 20 % at 8); 277 at 8 before a unit's elements were loaded at once and
+// diagonals of a tile shared an x window.  The random 1 M row matrix: 111 us
+// at 4 CTAs of 256, 122 at 3.  Variant 0 is the default; the format autotuner times all
+// four.
+constexpr int csb_ctas(int nt) { return nt == 128 ? 7 : 4; }
 constexpr int kCsbMaxS = 1024;
 constexpr int kDenseUnit = kTileDenseUnit;  // elements from which a unit's x window is staged
 
@@ -258,7 +263,7 @@ __device__ __forceinline__ void dense_oct(const Oct<K>& q, int S, const double* 
 // win_ptr[2w] = the window's first unit, win_ptr[2w+1] = its first dense
 // unit, win_ptr[2w+2] = the next window's first unit.
 template <int NT, int K>
-__global__ void __launch_bounds__(NT, kCsbThreadsPerSM / NT) k_csb_spmv(const uint32_t* __restrict__ ind, const int32_t* __restrict__ kcol, const double* __restrict__ data,
+__global__ void __launch_bounds__(NT, csb_ctas(NT)) k_csb_spmv(const uint32_t* __restrict__ ind, const int32_t* __restrict__ kcol, const double* __restrict__ data,
                                                      const int* __restrict__ win_ptr, const int4* __restrict__ units,
                                                      int nwin, int S, int nor, int noc, const double* __restrict__ x,
                                                      double* __restrict__ y, const double* nsq_in, int* status) {
@@ -267,25 +272,23 @@ __global__ void __launch_bounds__(NT, kCsbThreadsPerSM / NT) k_csb_spmv(const ui
     __shared__ __align__(8) uint64_t bar[2];
     const int tid = threadIdx.x;
     const int e = nsq_in ? pow2_rescale_exponent(*nsq_in, 256) : 0;
-    const bool tma_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    const uint64_t pol = policy_evict_normal();
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         fence_mbar_init();
     }
     __syncthreads();
-    uint32_t uses[2] = {0u, 0u};  // completed phases per buffer (same in every thread)
+    uint32_t n = 0u;  // x windows landed (same in every thread); window i uses buffer i & 1
     // stage the x window of unit u into buffer b (thread 0: TMA bulk copy;
     // the odd last element, if any, with a plain load)
     auto stage = [&](int u, int b) {
         const int c0 = __ldg(&units[u].z);
         const int cnt = min(S, noc - c0);
-        if (tma_ok) {
+        if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
             if (tid == 0) {
                 const uint32_t bytes = (uint32_t)(cnt & ~1) * 8u;
                 mbar_arrive_expect_tx(&bar[b], bytes);
-                if (bytes) bulk_g2s(xs[b], x + c0, bytes, &bar[b], pol);
+                if (bytes) bulk_g2s(xs[b], x + c0, bytes, &bar[b], policy_evict_normal());
                 if (cnt & 1) xs[b][cnt - 1] = __ldg(x + c0 + cnt - 1);
             }
         } else {
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(NT, kCsbThreadsPerSM / NT) k_csb_spmv(const ui
     for (int w = blockIdx.x; w < nwin; w += gridDim.x) {
         const int us = __ldg(win_ptr + 2 * w), u0 = __ldg(win_ptr + 2 * w + 1), u1 = __ldg(win_ptr + 2 * w + 2);
         for (int i = tid; i < S; i += NT) ys[i] = 0.0;
-        if (u0 < u1) stage(u0, 0);
+        if (u0 < u1) stage(u0, n & 1);
         __syncthreads();  // ys zeroed
         // the window's sparse sub-squares as one flat row-major unit, x
         // gathered through L1 / L2 by global column
@@ -312,56 +315,64 @@ __global__ void __launch_bounds__(NT, kCsbThreadsPerSM / NT) k_csb_spmv(const ui
         }
         bool ok = true;
         for (int u = u0; u < u1; ++u) {
-            const int b = (u - u0) & 1;
-            __syncthreads();  // buffer b^1 is free (its unit is done), ys zeroed
-            if (u + 1 < u1) stage(u + 1, b ^ 1);
             const int4 un = __ldg(units + u);
+            // a new x window (diagonals of one tile share theirs)
+            const bool fresh = u == u0 || __ldg(&units[u - 1].z) != un.z;
+            // ys holds the units before; the x window before is free, so the
+            // next one lands there
+            auto turn = [&]() {
+                __syncthreads();
+                if (!fresh) return;
+                int ahead = u + 1;
+                while (ahead < u1 && __ldg(&units[ahead].z) == un.z) ++ahead;
+                if (ahead < u1) stage(ahead, (n + 1) & 1);
+            };
+            auto landed = [&]() {
+                if (!fresh) return true;
+                ok = mbar_wait_bounded(&bar[n & 1], n >> 1 & 1u, status);
+                ok = __syncthreads_and(ok);
+                ++n;
+                return ok;
+            };
             if (un.w == 2) {
-                // one element per row: element lo + i to lane i % 32 of warp
-                // (i / 32) % W, so a warp's loads, x-window reads and y-window
-                // updates are 32 consecutive rows (no bank conflicts), four
-                // elements per lane in flight (the first four while the x
-                // window lands); one FMA per element from the row's y-window
-                // value
-                uint32_t id[4];
-                double v[4];
-                int base = un.x + warp * 128;
-                auto load4 = [&](int bs) {
+                // one element per row (at most S of them): element lo + i to
+                // lane i % 32 of a warp, so a warp's loads, x-window reads and
+                // y-window updates are 32 consecutive rows (no bank
+                // conflicts), U per lane in flight while the x window lands;
+                // one FMA per element from the row's y-window value
+                constexpr int U = kCsbMaxS / NT;
+                uint32_t id[U];
+                double v[U], acc[U];
+                const int k0 = un.x + warp * (32 * U) + lane;
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const int k = bs + 32 * t + lane;
-                        id[t] = k < un.y ? __ldg(ind + k) : 0u;
-                        v[t] = k < un.y ? __ldg(data + k) : 0.0;
-                    }
-                };
-                load4(base);
-                ok = mbar_wait_bounded(&bar[b], uses[b] & 1u, status);
-                uses[b]++;
-                if (!__syncthreads_and(ok)) break;
-                const double* xw = xs[b];
-                while (base < un.y) {
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        if (base + 32 * t + lane < un.y) {
-                            const int r = (int)(id[t] >> 16) & (S - 1);
-                            ys[r] = fma(v[t], xw[id[t] & (uint32_t)(S - 1)], ys[r]);
-                        }
-                    }
-                    base += (NT / 32) * 128;
-                    if (base < un.y) load4(base);
+                for (int t = 0; t < U; ++t) {
+                    const bool in = k0 + 32 * t < un.y;
+                    id[t] = in ? __ldcs(ind + k0 + 32 * t) : 0u;
+                    v[t] = in ? __ldcs(data + k0 + 32 * t) : 0.0;
                 }
+                turn();
+                if (!landed()) break;
+                const double* xw = xs[(n - 1) & 1];
+#pragma unroll
+                for (int t = 0; t < U; ++t)
+                    if (k0 + 32 * t < un.y) acc[t] = ys[(int)(id[t] >> 16) & (S - 1)];
+#pragma unroll
+                for (int t = 0; t < U; ++t)
+                    if (k0 + 32 * t < un.y) acc[t] = fma(v[t], xw[id[t] & (uint32_t)(S - 1)], acc[t]);
+#pragma unroll
+                for (int t = 0; t < U; ++t)
+                    if (k0 + 32 * t < un.y) ys[(int)(id[t] >> 16) & (S - 1)] = acc[t];
                 continue;
             }
             // row-major unit: warp chunks of kChunk elements; the first
             // chunk's loads are in flight while the x window lands
+            turn();
             constexpr int kChunk = 32 * K;
             constexpr int kStep = (NT / 32) * kChunk;
             int k = un.x + warp * kChunk;
             Oct<K> q = load_oct<K, false>(ind, kcol, data, k, un.x, un.y, S, lane);
-            ok = mbar_wait_bounded(&bar[b], uses[b] & 1u, status);
-            uses[b]++;
-            if (!__syncthreads_and(ok)) break;
-            const double* xw = xs[b];
+            if (!landed()) break;
+            const double* xw = xs[(n - 1) & 1];
             while (k < un.y) {
                 dense_oct<K, false>(q, S, xw, nullptr, ys, lane);
                 k += kStep;
@@ -371,7 +382,8 @@ __global__ void __launch_bounds__(NT, kCsbThreadsPerSM / NT) k_csb_spmv(const ui
         if (!ok) {
             // a wait timed out: let the copies in flight land, then stop
             if (tid == 0)
-                for (int b = 0; b < 2; ++b) mbar_wait_bounded(&bar[b], uses[b] & 1u, status, kWaitCycles / 8, false);
+                for (uint32_t i = n - 1; i != n + 1; ++i)
+                    mbar_wait_bounded(&bar[i & 1], i >> 1 & 1u, status, kWaitCycles / 8, false);
             __syncthreads();
             return;
         }
@@ -677,7 +689,11 @@ cudaError_t launch_csb_spmv(const uint32_t* ind, const int32_t* kcol, const doub
     if (nwin <= 0) return cudaSuccess;
     const int4* un = reinterpret_cast<const int4*>(units);
     const int nt = (variant & 2) ? 256 : 128;
-    const int grid = std::min(nwin, sm_count * (kCsbThreadsPerSM / nt));
+    // 256 threads (irregular matrices): a CTA per window, so the block
+    // scheduler evens out windows of unequal work (random 1 M rows: 111 us,
+    // 114 with resident CTAs that stride over the windows); 128 threads
+    // (stencils, equal windows): resident CTAs (4096^2 Poisson 227 us, 231).
+    const int grid = nt == 256 ? nwin : std::min(nwin, sm_count * csb_ctas(nt));
     switch (variant & 3) {
         case 1: k_csb_spmv<128, 8><<<grid, 128, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
         case 2: k_csb_spmv<256, 4><<<grid, 256, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
