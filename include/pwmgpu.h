@@ -234,13 +234,14 @@ int pwmgpu_set_power_mode(pwmgpu_matrix* m, int mode);
 int pwmgpu_test_grid_wait(pwmgpu_matrix* m, int64_t cycles, int32_t extra);
 
 /* Storage the FP32 / BF16 iterations (pwmgpu_solve's low-precision phase,
- * pwmgpu_mv_device_f32) stream (not in the reference).  AUTO (default): a
+ * pwmgpu_mv_device_f32) stream (not in the reference).  AUTO (default): the
+ * matrix's diagonal slices or sorted rows where its load chose them, else a
  * SELL-32 copy (slices of 32 rows, one row per lane, 16-bit column offsets;
  * built on first use) for matrices whose columns all lie within 32768 rows
  * of their row's slice and whose padding is within a quarter of the
- * nonzeros -- stencils and banded matrices -- the merge-path layout
- * otherwise; MERGE: always the merge-path layout.  The SELL kernel sums each
- * row left to right in CRS order; results differ from the merge layout's
+ * nonzeros -- other banded matrices -- the merge-path layout otherwise;
+ * MERGE: always the merge-path layout.  Slices and SELL-32 sum each row left
+ * to right in CRS order (sorted rows: long ones in a fixed tree); results differ from the merge layout's
  * only by rounding (within the FP32 row bound either way).  The power modes
  * above apply to the merge layout; POWER_FUSED keeps the low-precision
  * iterations on it too. */
@@ -381,7 +382,9 @@ int pwmgpu_tile_layout_host(int32_t format, int32_t nor, int32_t noc, int64_t nn
  * matrix (prefer_l1: 0 = most resident CTAs, 1 = a smaller shared-memory
  * carveout leaving more L1 for the x gathers; both compute the same bits),
  * the SpMV and persistent-power grids, and the two timings compared
- * (tuned_ms[2], ms per SpMV; 0 when the matrix was too small to tune). */
+ * (tuned_ms[2], ms per SpMV; 0 when the matrix was too small to tune).  A
+ * matrix on slices runs the merge kernels under POWER_FUSED / LOWFMT_MERGE
+ * only; they are timed over a quarter of its sub-tiles. */
 int pwmgpu_launch_config(const pwmgpu_matrix* m, int32_t* prefer_l1, int32_t* grid, int32_t* power_grid,
                          float* tuned_ms);
 /* The merge kernels' full launch variant: bit 0 = the smaller shared-memory

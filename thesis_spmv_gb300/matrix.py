@@ -231,8 +231,8 @@ class CudaSparseMatrix:
         check(_lib.lib().pwmgpu_set_power_mode(self._h, int(mode)), "set_power_mode")
 
     def set_low_format(self, fmt):
-        """LOWFMT_AUTO (SELL-32 for the FP32 / BF16 iterations where the
-        matrix fits it) / LOWFMT_MERGE (always the merge-path layout)."""
+        """LOWFMT_AUTO (the matrix's slices for the FP32 / BF16 iterations, else
+        SELL-32 where it fits) / LOWFMT_MERGE (always the merge-path layout)."""
         check(_lib.lib().pwmgpu_set_low_format(self._h, int(fmt)), "set_low_format")
 
     def solve(self, x, max_it, tol, precision=PREC_F64):
