@@ -225,7 +225,9 @@ __global__ void __launch_bounds__(kDiagNT, kDiagOcc) k_diag_spmv(DiagArgs<VT, XT
         copy_commit();
         return q;
     };
-    // plan data: loaded before the kernel before on the stream has ended
+    // Plan data, loaded before the kernel before on the stream has ended: what
+    // stage_next reads (records, offsets, masks, values) was complete, its
+    // stream synchronised, before this launch was made.
     DiagGroup cur = stage_next(0);
     pdl_wait();
     int e = 0;
@@ -407,7 +409,13 @@ int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st) {
         k_diag_convert<__nv_bfloat16><<<8 * sm_count, 256, 0, st>>>(D.val64, (__nv_bfloat16*)D.valbf, (size_t)D.elems);
     else
         k_diag_convert<float><<<8 * sm_count, 256, 0, st>>>(D.val64, D.val32, (size_t)D.elems);
-    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    // k_diag_spmv stages its first values before it waits for the kernel
+    // before it, so they are complete before a product can be launched
+    if (cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) return 0;
+    (void)cudaGetLastError();
+    dev_free(*dst);
+    *dst = nullptr;
+    return 2;
 }
 
 cudaError_t launch_diag_maxcol(const DiagPlan& D, int nor, int noc, int K, int* out, cudaStream_t st) {

@@ -122,6 +122,8 @@ struct DiagPlan {
 // no memory (D stays empty).
 int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
                int sm_count, cudaStream_t st);
+// The values in FP32 / BF16, made on first use and complete on return (the
+// stream is synchronised: not inside a capture).  0, or 2 as diag_build.
 int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st);
 // One pass over slices [c0, c1) (c1 < 0: all).  mode kModeSpmv: y = A x;
 // kModePower: y = 2^e A x and *nsq_out = ||y||^2 (when given; counter zero
@@ -165,6 +167,7 @@ struct RowsPlan {
 // stays empty).
 int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
                bool narrow, int sm_count, cudaStream_t st);
+// As diag_low_values.
 int rows_low_values(RowsPlan& R, bool bf16, int sm_count, cudaStream_t st);
 // Pipelined host-array SpMV: out[w] = the largest column of windows 0 .. w.
 cudaError_t launch_rows_maxcol(const RowsPlan& R, int* out, cudaStream_t st);

@@ -432,7 +432,11 @@ int rows_low_values(RowsPlan& R, bool bf16, int sm_count, cudaStream_t st) {
         k_rows_convert<__nv_bfloat16><<<8 * sm_count, 256, 0, st>>>(R.val64, (__nv_bfloat16*)R.valbf, (size_t)R.elems);
     else
         k_rows_convert<float><<<8 * sm_count, 256, 0, st>>>(R.val64, R.val32, (size_t)R.elems);
-    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    if (cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) return 0;
+    (void)cudaGetLastError();
+    dev_free(*dst);
+    *dst = nullptr;
+    return 2;
 }
 
 cudaError_t launch_rows_maxcol(const RowsPlan& R, int* out, cudaStream_t st) {
