@@ -1,0 +1,122 @@
+"""A handle's device memory outlives the work that uses it, also work the
+handle cannot know of: a graph captured from its stream and replayed on
+another one.  Loading another matrix into the handle, or dropping it, returns
+only when replays already enqueued have ended.  Handles on several host
+threads; the pool's memory goes back to the device with the last handle."""
+import os
+import subprocess
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _stencil(pwm):
+    M = pwm.CRSCuda(1)
+    M.generatePoissonMatrix(2048, 2048, 1)
+    return M
+
+
+def _irregular(pwm):
+    M = pwm.CRSCuda(1)
+    M.generateRandom(1_000_000, 5, mean_len=16.0)
+    return M
+
+
+@pytest.mark.parametrize("end", ["load", "drop"])
+@pytest.mark.parametrize("kind", ["stencil", "irregular"])
+def test_replays_end_before_the_memory_goes_back(kind, end):
+    torch = pytest.importorskip("torch")
+    import thesis_spmv_gb300 as pwm
+    M = (_stencil if kind == "stencil" else _irregular)(pwm)
+    n = M.dims()[0]
+    x = torch.rand(n, dtype=torch.float64, device="cuda")
+    want, y = torch.empty_like(x), torch.zeros_like(x)
+    torch.cuda.synchronize()
+    M.mv_device(x.data_ptr(), want.data_ptr())
+    torch.cuda.synchronize()
+    own, other = torch.cuda.Stream(), torch.cuda.Stream()
+    M.set_stream(own.cuda_stream)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=own):
+        for _ in range(20):
+            M.mv_device(x.data_ptr(), y.data_ptr())
+    done = torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        for _ in range(40):  # some 30 ms of products
+            g.replay()
+        done.record()
+    if end == "load":
+        M.generatePoissonMatrix(9, 9, 1)
+    else:
+        del M
+    assert done.query()
+    assert torch.equal(y, want)
+    if end == "load":
+        A = O.fill_poisson(9, 9)
+        v, u = np.random.default_rng(1).random(81), np.zeros(81)
+        M.mv(v, u)
+        assert np.all(np.abs(u - O.crs_mv(A, v)) <= O.row_error_bound(A, v))
+        M.set_stream(0)
+    torch.cuda.synchronize()
+
+
+def test_handles_on_several_threads():
+    """Loads, products, power steps whose buffers grow, and drops side by side."""
+    import thesis_spmv_gb300 as pwm
+    failed = []
+
+    def work(k):
+        rng = np.random.default_rng(k)
+        try:
+            for i in range(6):
+                M = pwm.CRSCuda(1)
+                for m in (5 + 9 * k, 40 + 31 * i, 211):
+                    A = O.fill_poisson(m, m + 3)
+                    M.generatePoissonMatrix(m, m + 3, 1)
+                    x, y = rng.random(A.nor), np.zeros(A.nor)
+                    M.mv(x, y)
+                    assert np.all(np.abs(y - O.crs_mv(A, x)) <= O.row_error_bound(A, x))
+                    it = 3 + 40 * i
+                    xg, yg = x.copy(), np.zeros(A.nor)
+                    M.powerIteration(xg, yg, it)
+                    xr, yr = O.power(A, x, it)
+                    np.testing.assert_allclose(yg, yr, rtol=1e-10, atol=1e-13)
+                del M
+        except Exception as e:  # noqa: BLE001 (reported by the test's thread)
+            failed.append(e)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not failed, failed[0]
+
+
+POOL = """
+import torch, thesis_spmv_gb300 as pwm
+M = pwm.CRSCuda(1)
+del M
+torch.cuda.synchronize()
+free0 = torch.cuda.mem_get_info()[0]
+A = pwm.CRSCuda(1); A.generatePoissonMatrix(2048, 2048, 1)
+B = pwm.CRSCuda(1); B.generatePoissonMatrix(64, 48, 1)
+assert torch.cuda.mem_get_info()[0] < free0 - (200 << 20)
+del A, B
+assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20), (free0, torch.cuda.mem_get_info())
+print("ok")
+"""
+
+
+def test_pool_goes_back_with_the_last_handle():
+    """(in a process of its own: other tests' handles would keep the pool)"""
+    r = subprocess.run([sys.executable, "-c", POOL], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr

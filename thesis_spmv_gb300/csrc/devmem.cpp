@@ -13,12 +13,17 @@
 // and an allocation that fails empties the pool and tries again.  The pool's
 // stream only orders allocations: a block is ready on every stream when
 // dev_alloc returns, and dev_free, unlike cudaFree, waits for nothing -- its
-// callers have synchronised the work that used the block.  Both may be called
+// callers have synchronised the work that used the block.  A handle cannot
+// know all the work that uses its blocks (a graph captured from its stream may
+// be replayed on any other), so it frees them inside a DevIdle scope, which
+// waits for the device first, as cudaFree did.  All of these may be called
 // from any thread.
 #include <cuda_runtime.h>
 
 #include <map>
 #include <mutex>
+#include <new>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -39,6 +44,13 @@ std::map<int, Pool>& pools() {
     static auto* p = new std::map<int, Pool>();
     return *p;
 }
+
+// Blocks freed where the device could not be waited for: {device, block}.
+std::vector<std::pair<int, void*>>& kept() {
+    static auto* p = new std::vector<std::pair<int, void*>>();
+    return *p;
+}
+thread_local int t_keep = 0;  // > 0: this thread's frees go to kept()
 
 // The pool of device `dev` (the current one), made on first use; null with
 // *e set when it cannot be made.  Call with g_mu held.
@@ -106,12 +118,53 @@ void dev_free(void* p) {
         return;
     }
     std::lock_guard<std::mutex> lk(g_mu);
+    if (t_keep > 0) {
+        try {
+            kept().emplace_back(a.device, p);
+        } catch (const std::bad_alloc&) {  // the block stays allocated
+        }
+        return;
+    }
     Pool& q = pools()[a.device];
     cudaFreeAsync(p, q.stream);
     if (--q.live == 0) {
         cudaStreamSynchronize(q.stream);
         cudaMemPoolTrimTo(q.pool, 0);
     }
+}
+
+DevIdle::DevIdle(int device) {
+    int cur = device;
+    (void)cudaGetDevice(&cur);
+    if (cur != device) (void)cudaSetDevice(device);
+    refused_ = cudaDeviceSynchronize() != cudaSuccess;
+    if (cur != device) (void)cudaSetDevice(cur);
+    if (refused_) {
+        (void)cudaGetLastError();
+        ++t_keep;
+        return;
+    }
+    std::vector<std::pair<int, void*>> back;  // what earlier scopes could not wait for
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (kept().empty()) return;
+        back.swap(kept());
+    }
+    for (auto& b : back) {
+        if (b.first == device && t_keep == 0) {
+            dev_free(b.second);
+            continue;
+        }
+        std::lock_guard<std::mutex> lk(g_mu);
+        try {
+            kept().push_back(b);
+        } catch (const std::bad_alloc&) {
+        }
+    }
+}
+
+DevIdle::~DevIdle() {
+    if (refused_) --t_keep;
 }
 
 size_t dev_idle_bytes() {

@@ -50,6 +50,20 @@ struct MergeGeom {
 // used the block has been synchronised before.
 cudaError_t dev_alloc(void** out, size_t bytes);
 void dev_free(void* p);
+// Waits for all work on `device` (as cudaFree does), so that blocks whose users
+// are not all known can be freed inside the scope.  Where the wait is refused
+// (a stream is being captured), the scope's dev_free calls keep their blocks
+// until a later scope's wait succeeds.
+class DevIdle {
+public:
+    explicit DevIdle(int device);
+    ~DevIdle();
+    DevIdle(const DevIdle&) = delete;
+    DevIdle& operator=(const DevIdle&) = delete;
+
+private:
+    bool refused_ = false;
+};
 // Bytes the current device's pool holds without using them.
 size_t dev_idle_bytes();
 // A pinned host block of 128 bytes.

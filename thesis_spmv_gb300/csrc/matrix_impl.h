@@ -189,9 +189,20 @@ struct pwmgpu_matrix {
         pwmgpu::dfree(coh.units);
         coh = decltype(coh)();
     }
-    // (the buffers go back without a wait: the handle's work ends first)
+    // The work that uses the buffers ends before they go back: the device's,
+    // because graphs captured from the handle's stream may run on any other.
+    // (A serving loop's matrix has no such users, and the loop frees it
+    // between rounds, with the other solves' work under way.)
     void release_matrix() {
-        cudaStreamSynchronize(stream);
+        if (batched) {
+            cudaStreamSynchronize(stream);
+            drop_matrix();
+        } else {
+            pwmgpu::DevIdle idle(device);
+            drop_matrix();
+        }
+    }
+    void drop_matrix() {
         for (void* p : outgrown) pwmgpu::dev_free(p);
         outgrown.clear();
         pwmgpu::dfree(M.row_start);
@@ -224,7 +235,16 @@ struct pwmgpu_matrix {
         loaded = false;
     }
     void release_all() {
-        release_matrix();
+        if (batched) {
+            cudaStreamSynchronize(stream);
+            drop_all();
+        } else {
+            pwmgpu::DevIdle idle(device);
+            drop_all();
+        }
+    }
+    void drop_all() {
+        drop_matrix();
         for (cudaEvent_t e : pipe.ev_x) cudaEventDestroy(e);
         for (cudaEvent_t e : pipe.ev_y) cudaEventDestroy(e);
         if (pipe.ev_start) cudaEventDestroy(pipe.ev_start);

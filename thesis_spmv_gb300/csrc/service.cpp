@@ -118,9 +118,11 @@ struct ClassDev {
     size_t grp_cap = 0;
 };
 
-int grow(double** p, size_t* cap, size_t need) {
+// (a round that a failed step left under way may use the old buffer)
+int grow(int device, double** p, size_t* cap, size_t need) {
     if (*cap >= need && *p) return PWMGPU_OK;
     size_t c = std::max(need, *cap * 2);
+    DevIdle idle(device);
     dfree(*p);
     *cap = 0;
     TRY(dalloc(p, c));
@@ -174,6 +176,7 @@ struct pwmsvc {
     double now() const { return std::chrono::duration<double>(Clock::now() - t0).count(); }
 
     void release() {
+        DevIdle idle(device);  // rounds that a failed step left under way end first
         for (auto& kv : all)
             if (kv.second->m) pwmgpu_destroy(kv.second->m);
         for (auto& g : graphs) {
@@ -334,21 +337,23 @@ int rebuild_tables(pwmsvc* S) {
         if (hs.empty()) continue;  // not in the round
         S->mask |= 1u << c;
         if (D.slots_cap < hs.size() || !D.d_slots) {
+            DevIdle idle(S->device);  // as grow()
             dfree(D.d_slots);
             D.slots_cap = 0;
             TRY(dalloc(&D.d_slots, std::max<size_t>(hs.size(), 64)));
             D.slots_cap = std::max<size_t>(hs.size(), 64);
         }
         if (D.slot_cap < (size_t)tiles + 1 || !D.tile_slot) {
+            DevIdle idle(S->device);
             dfree(D.tile_slot);
             D.slot_cap = 0;
             const size_t cap = std::max<size_t>((size_t)tiles + 1, 2 * D.slot_cap);
             TRY(dalloc(&D.tile_slot, cap));
             D.slot_cap = cap;
         }
-        TRY(grow(&D.row_part, &D.row_cap, 2 * (size_t)rows + 2));
-        TRY(grow(&D.res_part, &D.res_cap, (size_t)rows + 1));
-        if (sell) TRY(grow(&D.grp_part, &D.grp_cap, (size_t)fix + 1));
+        TRY(grow(S->device, &D.row_part, &D.row_cap, 2 * (size_t)rows + 2));
+        TRY(grow(S->device, &D.res_part, &D.res_cap, (size_t)rows + 1));
+        if (sell) TRY(grow(S->device, &D.grp_part, &D.grp_cap, (size_t)fix + 1));
         CU(cudaMemcpyAsync(D.d_slots, hs.data(), hs.size() * sizeof(BatchSlot), cudaMemcpyHostToDevice, S->stream));
         BatchTable T{};
         T.nslots = (int)hs.size();
