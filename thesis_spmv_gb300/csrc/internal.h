@@ -314,10 +314,17 @@ struct TripletScan {
 };
 cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long long nnz, int32_t nor, int32_t noc,
                                 int32_t* cnt, int32_t* pos, TripletScan* flags, int sm_count, cudaStream_t st);
-// Rows of at most `longest` entries can be sorted by launch_triplet_rows: CRS
-// from the row starts and the scan's arrival numbers pos (which receive the
+// The work of launch_triplet_rows on rows of these lengths.
+struct TripletWork {
+    unsigned long long sum, most;  // sums of squared row lengths: all rows', and the largest of a CTA's rows
+};
+// cnt: the row lengths.
+cudaError_t launch_triplet_work(const int32_t* cnt, int32_t nor, TripletWork* out, int sm_count, cudaStream_t st);
+// Whether launch_triplet_rows sorts the rows no slower than the radix sort (w
+// null: from the longest row alone; false then means perhaps).
+bool triplet_rows_fit(int longest, const TripletWork* w, long long nnz);
+// CRS from the row starts and the scan's arrival numbers pos (which receive the
 // sorted rows with rows_out); src: nnz words of scratch.
-bool triplet_rows_fit(int longest);
 cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
                                 long long nnz, const int32_t* row_start, int32_t nor, int32_t* src, int32_t* col,
                                 double* val, bool rows_out, int sm_count, cudaStream_t st);

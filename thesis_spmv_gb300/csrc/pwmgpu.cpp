@@ -1320,6 +1320,7 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
     int32_t* scan_scratch = nullptr;
     int32_t* pos = nullptr;
     TripletScan* dflags = nullptr;
+    TripletWork* dwork = nullptr;
     unsigned long long *keys_a = nullptr, *keys_b = nullptr;
     int32_t *src_a = nullptr, *src_b = nullptr, *tab = nullptr, *tab_scratch = nullptr;
     bool matrix_touched = false;
@@ -1349,6 +1350,18 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
                 rc = fail(PWMGPU_ERR_INVALID, "column %d at entry %lld out of range", c, k);
             break;
         }
+        // rows sorted in shared memory or all entries by radix
+        bool by_rows = flags.unsorted_rc && triplet_rows_fit(flags.longest, nullptr, nnz);
+        if (flags.unsorted_rc && !by_rows) {
+            TripletWork work{};
+            if ((rc = dalloc(&dwork, 1)) != PWMGPU_OK) break;
+            e = launch_triplet_work(cnt + 1, nor, dwork, m->sm_count, m->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(&work, dwork, sizeof work, cudaMemcpyDeviceToHost, m->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+            if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "triplet rows: %s", cudaGetErrorString(e)); break; }
+            by_rows = triplet_rows_fit(flags.longest, &work, nnz);
+        }
+        if (!by_rows) dfree(pos);
         e = launch_inclusive_scan(cnt + 1, nor, scan_scratch, m->stream);
         if (e != cudaSuccess) { rc = fail(PWMGPU_ERR_CUDA, "row scan: %s", cudaGetErrorString(e)); break; }
         matrix_touched = true;
@@ -1362,7 +1375,7 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(m->M.val, vals, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice,
                                     m->stream);
-        } else if (e == cudaSuccess && nnz > 0 && triplet_rows_fit(flags.longest)) {
+        } else if (e == cudaSuccess && nnz > 0 && by_rows) {
             if ((rc = dalloc(&src_a, (size_t)nnz)) != PWMGPU_OK) break;
             e = launch_triplet_rows(rows, cols, vals, pos, nnz, m->M.row_start, nor, src_a, m->M.col, m->M.val,
                                     h_rows != nullptr, m->sm_count, m->stream);
@@ -1402,6 +1415,7 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
     dfree(scan_scratch);
     dfree(pos);
     dfree(dflags);
+    dfree(dwork);
     dfree(keys_a);
     dfree(keys_b);
     dfree(src_a);

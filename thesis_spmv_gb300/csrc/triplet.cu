@@ -11,11 +11,11 @@
 //      returned), the longest row, and two order flags: "not sorted by (row,
 //      col)" and "not sorted by column".
 //   2. Already sorted by (row, col): col / val are the input, copied.
-//   3. Rows of at most kRowSortMax entries: k_trip_bucket writes each entry's
-//      index to row_start + arrival number, k_trip_rows sorts every row in
-//      shared memory by (column, index) -- an element's place is the number of
-//      smaller keys in its row, so the order of the arrivals does not matter
-//      -- and k_trip_vals gathers the values.  Bound by the row atomics, the
+//   3. Rows of at most kRowSortMax entries, where that pays (triplet_rows_fit):
+//      k_trip_bucket writes each entry's index to row_start + arrival number,
+//      k_trip_rows sorts every row in shared memory by (column, index) -- an
+//      element's place is the number of smaller keys in its row, so the order
+//      of the arrivals does not matter -- and k_trip_vals gathers the values.  Bound by the row atomics, the
 //      scattered stores and the two gathers; every other access is a stream.
 //      Scattered stores of 4 bytes run at 196 G/s, of 16 bytes at 31 G/s (67
 //      and 268 MB), gathers at 260 G/s from what L2 holds and 117 G/s from 134
@@ -25,7 +25,7 @@
 //      index, value} records, 2.80 so (scan 0.24 ms, bucket 0.26, rows 0.26,
 //      values 0.27); sorted by column 2.40 -> 2.23 ms; 8 M entries of a random
 //      matrix 1.34 -> 1.20.
-//   4. Longer rows: a stable LSD radix sort of the packed key row << 32 | col
+//   4. Otherwise: a stable LSD radix sort of the packed key row << 32 | col
 //      with 8-bit digits: first the column digits (skipped when the input is
 //      already sorted by column -- a stable sort by a key that is already in
 //      order is the identity), then the row digits.  Per pass: k_radix_hist
@@ -137,6 +137,29 @@ __global__ void __launch_bounds__(256) k_trip_bucket(const int32_t* __restrict__
             const long long k = k0 + u * step;
             if (k < nnz) src[at[u]] = (int32_t)k;
         }
+    }
+}
+
+// Compares k_trip_rows makes, a row's length squared each, from the row counts:
+// the sum, and the most of any kRowSortRows rows a CTA takes at a time.
+__global__ void __launch_bounds__(256) k_trip_work(const int32_t* __restrict__ cnt, int32_t nor, TripletWork* out) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long sum = 0, most = 0;
+    const long long blocks = ((long long)nor + kRowSortRows - 1) / kRowSortRows;
+    for (long long b = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); b < blocks; b += (long long)gridDim.x * 8) {
+        const long long r1 = min((long long)nor, (b + 1) * kRowSortRows);
+        unsigned long long t = 0;
+        for (long long r = b * kRowSortRows + lane; r < r1; r += 32) {
+            const unsigned long long n = (unsigned long long)__ldg(cnt + r);
+            t += n * n;
+        }
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        sum += t;
+        most = most > t ? most : t;
+    }
+    if (lane == 0 && most) {
+        atomicAdd(&out->sum, sum);
+        atomicMax(&out->most, most);
     }
 }
 
@@ -346,7 +369,29 @@ cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long l
     return cudaGetLastError();
 }
 
-bool triplet_rows_fit(int longest) { return longest <= kRowSortMax; }
+// k_trip_rows ranks an element against every key of its row, and a CTA takes
+// kRowSortRows rows: measured 33 ps per compare of one CTA, where the radix sort
+// takes some 40 us and 0.2 (row digits only) to 0.37 ns per entry.  So a CTA's
+// compares are held to what the radix sort does meanwhile, and all of them to
+// 1024 per entry (0.1 ns with the SMs busy).  Loads, all rows here and by this
+// rule: 512 x 4096 entries 288 and 1.6 ms, 2000 x 1000 18.6 and 1.4, 4096 x
+// 4096 290 and 8.4, 1 M rows of 4 around 512 of 1000 11.0 and 2.2; 100 000 x
+// 300 stays here (6.1 ms, radix sort 15.4).
+bool triplet_rows_fit(int longest, const TripletWork* w, long long nnz) {
+    const unsigned long long limit = (1ull << 20) + 4ull * (unsigned long long)nnz,
+                             row = (unsigned long long)longest * (unsigned long long)longest;
+    if (longest > kRowSortMax || row > limit) return false;
+    if (!w) return row * kRowSortRows <= limit && longest <= 1024;
+    return w->most <= limit && w->sum <= 1024ull * (unsigned long long)nnz;
+}
+
+cudaError_t launch_triplet_work(const int32_t* cnt, int32_t nor, TripletWork* out, int sm_count, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(TripletWork), st);
+    if (e != cudaSuccess) return e;
+    const long long ctas = ((long long)nor + 8 * kRowSortRows - 1) / (8 * kRowSortRows);
+    k_trip_work<<<(int)(ctas < 4LL * sm_count ? ctas : 4LL * sm_count), 256, 0, st>>>(cnt, nor, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_triplet_rows(const int32_t* rows, const int32_t* cols, const double* vals, int32_t* pos,
                                 long long nnz, const int32_t* row_start, int32_t nor, int32_t* src, int32_t* col,
