@@ -1,0 +1,98 @@
+"""Long rows of matrices on sorted rows: a warp does a row, so a row whose warp
+would still run when the rest is over starts in an earlier window of rows, and a
+matrix with a row too long for that stays on the merge path.  Values against
+the oracle wherever the long rows lie (FP64 rows within the oracle's row bound,
+FP32 rows within (2*nnz_row + 3) * 2^-24 * sum|a_ij x_j|), the bits of the
+chunked host-array product, and the time beside the same matrix without the row."""
+import numpy as np
+import pytest
+
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(lengths, noc, seed):
+    rng = np.random.default_rng(seed)
+    rs = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    return O.CRSArrays(len(lengths), noc, rs, rng.integers(0, noc, int(rs[-1])).astype(np.int32),
+                       rng.uniform(-1, 1, int(rs[-1])))
+
+
+def _at(n, short, at, long):
+    """n rows, `long` elements at the row numbers `at`, 0 .. 2 * short elsewhere."""
+    out = np.random.default_rng(n).integers(0, 2 * short + 1, n)
+    out[list(at)] = long
+    return out
+
+
+N = 300_001  # 16 windows of 18 751 rows
+CASES = {
+    "last": lambda: _at(N, 16, [N - 1], 5800),
+    "last_too_long": lambda: _at(N, 16, [N - 1], 6200),
+    "every_window": lambda: _at(N, 16, range(18_750, N, 18_751), 3000),
+    "window_starts": lambda: _at(N, 16, range(0, N, 18_751), 1700),
+    "just_late": lambda: _at(N, 16, [N - 3, N - 2, N - 1], [512, 513, 700]),
+    "one_window": lambda: _at(200_000, 16, [0, 100_000, 199_999], 4000),
+    "253_254_255": lambda: np.random.default_rng(1).choice([253, 254, 255, 63, 64, 65], 60_000),
+}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_long_rows(case):
+    torch = pytest.importorskip("torch")
+    import thesis_spmv_gb300 as pwm
+    A = _matrix(CASES[case](), N, 2)
+    M = pwm.CRSCuda(1)
+    M.loadCSR(A.nor, A.noc, A.row_start, A.col_ind, A.data)
+    x = np.random.default_rng(3).uniform(-1, 1, A.noc)
+    want, bound = O.crs_mv(A, x), O.row_error_bound(A, x)
+    y = np.full(A.nor, np.nan)
+    M.mv(x, y)  # 16 chunks where the matrix has 16 windows
+    assert np.all(np.abs(y - want) <= bound)
+    dx = torch.tensor(x, device="cuda")
+    dy = torch.full((A.nor,), float("nan"), dtype=torch.float64, device="cuda")
+    dx32, dy32 = dx.float(), dy.float()
+    torch.cuda.synchronize()
+    M.mv_device(dx.data_ptr(), dy.data_ptr())
+    M.mv_device_f32(dx32.data_ptr(), dy32.data_ptr())
+    torch.cuda.synchronize()
+    assert np.array_equal(dy.cpu().numpy(), y)
+    s = O.crs_mv(O.CRSArrays(A.nor, A.noc, A.row_start, A.col_ind, np.abs(A.data)), np.abs(x))
+    f32 = (2 * np.diff(A.row_start) + 3) * 2.0 ** -24 * s
+    assert np.all(np.abs(dy32.cpu().numpy().astype(np.float64) - want) <= f32)
+
+
+def _us(lengths):
+    torch = pytest.importorskip("torch")
+    import thesis_spmv_gb300 as pwm
+    A = _matrix(lengths, lengths.size, 4)
+    M = pwm.CRSCuda(1)
+    M.loadCSR(A.nor, A.noc, A.row_start, A.col_ind, A.data)
+    M.set_stream(torch.cuda.current_stream().cuda_stream)
+    x = torch.rand(A.noc, dtype=torch.float64, device="cuda")
+    y = torch.empty(A.nor, dtype=torch.float64, device="cuda")
+    best = 1e9
+    for _ in range(6):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        for _ in range(20):
+            M.mv_device(x.data_ptr(), y.data_ptr())
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) * 50)
+    return best
+
+
+@pytest.mark.parametrize("long", [9_000, 17_000])
+def test_a_long_last_row_costs_little(long):
+    """16.8 M elements without the row: 70 us.  A warp takes some 70 us for the
+    9000 elements and 127 us for the 17 000; begun after the other rows that
+    was a factor of 1.7 and more.  On the merge path the matrix takes 1.4 times
+    as long as without the row, so the bound lies at 1.55."""
+    n = 1 << 20
+    short = np.full(n, 16)
+    late = short.copy()
+    late[-1] = long
+    assert _us(late) <= 1.55 * _us(short)

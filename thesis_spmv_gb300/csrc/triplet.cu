@@ -373,10 +373,10 @@ cudaError_t launch_triplet_scan(const int32_t* rows, const int32_t* cols, long l
 // kRowSortRows rows: measured 33 ps per compare of one CTA, where the radix sort
 // takes some 40 us and 0.2 (row digits only) to 0.37 ns per entry.  So a CTA's
 // compares are held to what the radix sort does meanwhile, and all of them to
-// 1024 per entry (0.1 ns with the SMs busy).  Loads, all rows here and by this
-// rule: 512 x 4096 entries 288 and 1.6 ms, 2000 x 1000 18.6 and 1.4, 4096 x
-// 4096 290 and 8.4, 1 M rows of 4 around 512 of 1000 11.0 and 2.2; 100 000 x
-// 300 stays here (6.1 ms, radix sort 15.4).
+// 1024 per entry (0.1 ns with the SMs busy).  Loads with rows
+// of up to 4096 entries always here, and by this rule: 512 x 4096 entries 288
+// and 1.0 ms, 2000 x 1000 18.6 and 0.88, 4096 x 4096 290 and 3.4, 1 M rows of 4
+// around 512 of 1000 11.0 and 1.5; 100 000 x 300 stays here (6.1 ms).
 bool triplet_rows_fit(int longest, const TripletWork* w, long long nnz) {
     const unsigned long long limit = (1ull << 20) + 4ull * (unsigned long long)nnz,
                              row = (unsigned long long)longest * (unsigned long long)longest;
