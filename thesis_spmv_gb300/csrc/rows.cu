@@ -2,7 +2,8 @@
 // anywhere.
 //
 // Rows are sorted by length (longest first, equal lengths in row order;
-// within each of up to 16 windows of consecutive rows) and cut into items, a
+// within each of up to 16 windows of consecutive rows, a late window's longest
+// rows in an earlier one) and cut into items, a
 // warp's work: 32 rows with a lane each, 8 rows with four lanes each, or one
 // row with the whole warp, by length.  An item is a run of units of 64
 // (column, value) pairs: in unit j a lane with G lanes to its row holds the
@@ -23,7 +24,8 @@
 // 9.4 -> 5.1 us.  Twenty power steps on 1 M rows: 2.14 -> 1.60 ms.
 //
 // Windows keep a chunk of rows (and the y they store) together: a host-array
-// product sends a window's rows home while the next one runs.
+// product sends a window's rows home while the next one runs.  (A row that
+// moved to an earlier window is stored before it is sent.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -42,11 +44,13 @@ constexpr int kRowsOcc = 10;        // 48 registers
 constexpr int kRowsU = 3;           // units whose loads are issued together
 constexpr int kRowsWindows = 16;    // at most
 
-// The windows of a matrix and the lengths from which a row gets four lanes
-// (t4) and a warp (t32 <= 255).
+// The windows of a matrix, the lengths from which a row gets four lanes (t4)
+// and a warp (t32 <= 254) and goes before the other rows of its window (first
+// >= t32), and the elements by which a row beyond kRowsLate moves one window up.
 struct RowsCut {
-    int windows, wrows, t4, t32;
+    int windows, wrows, t4, t32, first, up;
 };
+constexpr int kRowsLate = 512;  // elements of a row that may start last
 // Rows of each window by class (0: a warp, 1: four lanes, 2: a lane each), the
 // longest row, and the units of all items (summed later).
 // And where each (window, class) starts, in items and in sorted rows.
@@ -58,7 +62,15 @@ struct RowsHead {
 };
 __host__ __device__ constexpr int class_shift(int cls) { return cls == 0 ? 5 : cls == 1 ? 2 : 0; }  // log2 of G
 
-// Sort key of a row: its window above a byte that puts long rows first.
+// The window in whose items a row runs: its own, or an earlier one where the
+// work from its own window on is over before a warp has done the row.
+__device__ __forceinline__ int row_window(int r, int len, const RowsCut& cut) {
+    const int back = len > kRowsLate ? (len - kRowsLate) / cut.up : 0;
+    return min(r / cut.wrows, max(cut.windows - 1 - back, 0));
+}
+
+// Sort key of a row: its window above a byte that puts long rows first (0: from
+// cut.first on; lengths below 254 each have a value of their own).
 __global__ void __launch_bounds__(256) k_rows_keys(const int32_t* __restrict__ row_start, int nor, RowsCut cut,
                                                    unsigned long long* __restrict__ key, int32_t* __restrict__ row,
                                                    RowsHead* head) {
@@ -67,8 +79,8 @@ __global__ void __launch_bounds__(256) k_rows_keys(const int32_t* __restrict__ r
     __syncthreads();
     int longest = 0;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nor; r += gridDim.x * blockDim.x) {
-        const int len = row_start[r + 1] - row_start[r], w = r / cut.wrows;
-        key[r] = (unsigned long long)w << 8 | (unsigned long long)(255 - min(len, 255));
+        const int len = row_start[r + 1] - row_start[r], w = row_window(r, len, cut);
+        key[r] = (unsigned long long)w << 8 | (unsigned long long)(len >= cut.first ? 0 : 255 - min(len, 254));
         row[r] = r;
         atomicAdd(&cnt[3 * w + (len >= cut.t32 ? 0 : len >= cut.t4 ? 1 : 2)], 1);
         longest = max(longest, len);
@@ -318,7 +330,7 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
     // matrix (little work beside its longest items) cuts earlier.  64 / 255
     // and 16 / 64: 30.5 and 27.5 us on 4.8 M nonzeros, 9.8 and 5.1 us on
     // 0.24 M; on 67 M nonzeros 64 / 255 beat 128 / 255 and 32 / 255 by 3 %.
-    RowsCut cut{1, nor, 64, 255};
+    RowsCut cut{1, nor, 64, 254, 0, 0};
     if (nnz < (1LL << 23)) {
         cut.t4 = 16;
         cut.t32 = 64;
@@ -327,6 +339,11 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
         cut.windows = kRowsWindows;
         cut.wrows = (nor + kRowsWindows - 1) / kRowsWindows;
     }
+    // A warp does 2000 elements of a row while the matrix does a million (7.5 ns
+    // and 4 ps an element): what a row has beyond kRowsLate runs beside the
+    // windows from its own on, or moves up to a window with as much behind it.
+    cut.up = (int)std::max(1LL, nnz / (2000LL * cut.windows));
+    cut.first = kRowsLate + (int)(nnz / 32000);
     RowsHead h{};
     auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
     const long long most = (long long)nor + 3 * kRowsWindows;  // items at most
@@ -364,10 +381,16 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
         if (launch_inclusive_scan(off + 1, most, scratch, st) != cudaSuccess) break;
         if (cudaMemcpyAsync(&h, dh, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess) break;
         if (cudaStreamSynchronize(st) != cudaSuccess) break;
-        // A row is one warp's work: 1024 elements take as long as a small
-        // matrix does on the merge path, a thousandth of the nonzeros as long
-        // as the rest of a large one.  Padding: as the merge layout's extra.
-        if ((double)h.longest > 1024.0 + (double)nnz / 1000.0 || h.units >= (1ull << 31) ||
+        // A row is one warp's work, 4.2 ns an element where L2 holds the matrix
+        // and 7.5 where it does not: 1024 elements take as long as a small
+        // matrix does on the merge path, a thousandth of the nonzeros as long as
+        // the rest of one in L2 (4.8 M, longest row 2400: 28 us, merge path 50),
+        // and a quarter of that is half of the rest of a large one.  (Longer
+        // ones: 60 000 elements in 67 M 450 us, 560 where the row came last,
+        // merge path 351; 17 000 in 16.7 M 134 and 102; eight of 10 000 in 9.5 M
+        // 85 and 66.)  Padding: as the merge layout's extra.
+        if ((double)h.longest > 1024.0 + std::min((double)nnz / 1000.0, 4096.0 + (double)nnz / 4000.0) ||
+            h.units >= (1ull << 31) ||
             (double)h.units * 64.0 > 1.25 * (double)nnz + 16384.0) {
             rc = 1;
             break;
