@@ -383,8 +383,9 @@ int pwmgpu_tile_layout_host(int32_t format, int32_t nor, int32_t noc, int64_t nn
  * carveout leaving more L1 for the x gathers; both compute the same bits),
  * the SpMV and persistent-power grids, and the two timings compared
  * (tuned_ms[2], ms per SpMV; 0 when the matrix was too small to tune).  A
- * matrix on slices runs the merge kernels under POWER_FUSED / LOWFMT_MERGE
- * only; they are timed over a quarter of its sub-tiles. */
+ * matrix on slices runs the merge kernels only under POWER_FUSED /
+ * LOWFMT_MERGE or once pwmgpu_set_launch_variant asks for them; they are timed
+ * over a quarter of its sub-tiles. */
 int pwmgpu_launch_config(const pwmgpu_matrix* m, int32_t* prefer_l1, int32_t* grid, int32_t* power_grid,
                          float* tuned_ms);
 /* The merge kernels' full launch variant: bit 0 = the smaller shared-memory
@@ -392,8 +393,19 @@ int pwmgpu_launch_config(const pwmgpu_matrix* m, int32_t* prefer_l1, int32_t* gr
 int pwmgpu_launch_variant(const pwmgpu_matrix* m, int32_t* variant);
 /* Override the tuner's choice for later launches: 0 or 1 (carveout), 4 or 5
  * (the same with x gathers that bypass L1, on FP64 iterations).  16-bit
- * columns are used wherever the plan has them. */
+ * columns are used wherever the plan has them.  A matrix on slices then runs
+ * on the merge kernels, in every precision, until the next load. */
 int pwmgpu_set_launch_variant(pwmgpu_matrix* m, int32_t variant);
+/* The layout the handle's products run on (no reference counterpart):
+ * precision PWMGPU_PREC_F64, or PWMGPU_PREC_F32 (pwmgpu_mv_device_f32; the FP32
+ * copies are made by the first such call, so ask after it). */
+#define PWMGPU_LAYOUT_MERGE 0     /* merge-path sub-tiles */
+#define PWMGPU_LAYOUT_DIAGONALS 1 /* diagonal slices */
+#define PWMGPU_LAYOUT_ROWS 2      /* sorted rows */
+#define PWMGPU_LAYOUT_SELL 3      /* SELL-32 */
+#define PWMGPU_LAYOUT_CSB 4
+#define PWMGPU_LAYOUT_COH 5
+int pwmgpu_layout(const pwmgpu_matrix* m, int precision, int32_t* layout);
 /* Bytes per column index the merge kernels stream: 2 when every merge
  * sub-tile's columns span less than 2^16 (banded and stencil matrices: the
  * plan then keeps 16-bit offsets from a per-sub-tile base), else 4; and

@@ -20,6 +20,7 @@ FMT_MERGE, FMT_CSB, FMT_COH, FMT_AUTO = 0, 1, 2, 3
 PREC_F64, PREC_F32, PREC_MIXED = 0, 1, 2
 POWER_AUTO, POWER_FUSED, POWER_MULTI = 0, 1, 2
 LOWFMT_AUTO, LOWFMT_MERGE = 0, 1
+LAYOUTS = ("merge", "diagonals", "rows", "sell", "csb", "coh")  # PWMGPU_LAYOUT_*
 RAND_LOGNORMAL, RAND_POISSON = 0, 1
 
 
@@ -103,6 +104,7 @@ SIGNATURES = {
     "pwmgpu_launch_config": (C.c_int, [vp, C.POINTER(i32), C.POINTER(i32), C.POINTER(i32), C.POINTER(C.c_float)]),
     "pwmgpu_set_launch_variant": (C.c_int, [vp, i32]),
     "pwmgpu_launch_variant": (C.c_int, [vp, C.POINTER(i32)]),
+    "pwmgpu_layout": (C.c_int, [vp, C.c_int, C.POINTER(i32)]),
     "pwmgpu_plan_info": (C.c_int, [vp, C.POINTER(i32), C.POINTER(i32)]),
     "pwmgpu_csb_build_host": (C.c_int, [i32, i32, i64, vp, vp, vp, vp, vp, vp]),
     "pwmgpu_coh_build_host": (C.c_int, [i32, i32, i64, vp, vp, vp, i32, C.POINTER(i32), C.POINTER(i64),

@@ -102,6 +102,9 @@ struct pwmgpu_matrix {
     // diagonal slices (nslices 0: the matrix does not fit them)
     pwmgpu::DiagPlan diag;
     pwmgpu::RowsPlan rows;  // sorted row slices (nitems 0: not built)
+    // a launch variant of the merge kernels was asked for: they run, not the
+    // slices, until the next load
+    bool merge_only = false;
 
     // scratch
     double* carries = nullptr;  // max(num_tiles, num_tiles32) doubles (also used as floats)
@@ -230,6 +233,7 @@ struct pwmgpu_matrix {
         sell.release();
         diag.release();
         rows.release();
+        merge_only = false;
         M = DevMatrix();
         num_tiles = 0;
         loaded = false;

@@ -81,6 +81,10 @@ namespace {
 namespace pwmgpu {
 // CSB / CO-H formats: build the format's arrays on the host from the CRS
 // arrays (which stay on the device for pwmgpu_get_csr), upload them.
+// A handle whose steps run on slices (diagonal ones, or sorted rows) rather
+// than the merge plan: one kernel per step, no fix-up.
+bool sliced(const pwmgpu_matrix* m) { return !m->merge_only && (m->diag.nslices || m->rows.nitems); }
+
 int build_format(pwmgpu_matrix* m) {
     const int nor = m->M.nor, noc = m->M.noc;
     const long long nnz = m->M.nnz;
@@ -193,7 +197,7 @@ int tune(pwmgpu_matrix* m) {
     // them: two timed runs over a quarter of the sub-tiles do (at least two
     // waves of CTAs).  Load of a 2048^2 stencil: 2.67 ms with two runs over
     // all of them, 2.18 so (the same variants chosen, stencils and irregular).
-    const bool side = m->diag.nslices || m->rows.nitems;
+    const bool side = sliced(m);
     const int reps = side ? 2 : 8, tiles = side ? m->num_tiles / 4 : m->num_tiles;
     for (int c = 0; c < 4 && rc == PWMGPU_OK; ++c) {
         const int v = cand[c] | c16;
@@ -422,10 +426,6 @@ int fp64_format(const pwmgpu_matrix* m) {
     if (m->format != PWMGPU_FMT_MERGE) return m->format;
     return m->tuned_fmt > 0 ? m->tuned_fmt : PWMGPU_FMT_MERGE;
 }
-
-// A handle whose steps run on slices (diagonal ones, or sorted rows) rather
-// than the merge plan: one kernel per step, no fix-up.
-bool sliced(const pwmgpu_matrix* m) { return m->diag.nslices || m->rows.nitems; }
 
 cudaError_t launch_sliced(pwmgpu_matrix* m, int cfg, int mode, const void* x, void* y, const SliceStep& s) {
     return m->diag.nslices ? launch_diag_spmv(m->diag, cfg, mode, m->M.nor, m->M.noc, x, y, s, m->sm_count, m->stream)
@@ -964,12 +964,12 @@ int plan_pipeline(pwmgpu_matrix* m) {
     p.K = -1;
     const int K = kPipeChunks;
     if (m->num_tiles < 64 * K) return PWMGPU_OK;  // too small to gain from it
-    const bool rows = m->rows.nitems > 0;
+    const bool rows = sliced(m) && m->rows.nitems > 0;
+    const bool diag = sliced(m) && m->diag.nslices > 0;
     if (rows && m->rows.windows != K) return PWMGPU_OK;
     int* d = nullptr;
     TRY(dalloc(&d, 4 * (size_t)K));
     p.rec.assign(4 * (size_t)K, 0);
-    const bool diag = m->diag.nslices > 0;
     cudaError_t e = diag ? launch_diag_maxcol(m->diag, m->M.nor, m->M.noc, K, d, m->stream)
                     : rows ? launch_rows_maxcol(m->rows, d, m->stream)
                            : launch_pipeline_plan(m->M.row_start, m->P, K, d, m->stream);
@@ -1041,7 +1041,7 @@ int mv_pipelined(pwmgpu_matrix* m, const double* x, double* y) {
     auto& p = m->pipe;
     const int K = p.K, noc = m->M.noc, nor = m->M.nor;
     const bool own = sliced(m);  // a chunk's rows are its own
-    const int nsub = m->diag.nslices ? m->diag.nslices : m->rows.nitems ? m->rows.nitems : m->num_tiles;
+    const int nsub = !own ? m->num_tiles : m->diag.nslices ? m->diag.nslices : m->rows.nitems;
     const bool x_sm = sm_reachable_pageable(m, x), y_sm = sm_reachable_pageable(m, y);
     // the streams start after earlier work on the handle's stream
     CU(cudaEventRecord(p.ev_start, m->stream));
@@ -2039,11 +2039,39 @@ int pwmgpu_set_launch_variant(pwmgpu_matrix* m, int32_t variant) {
         return fail(PWMGPU_ERR_INVALID, "launch variant must be 0, 1, 4 or 5");
     if (!m->loaded || m->format != PWMGPU_FMT_MERGE) return fail(PWMGPU_ERR_STATE, "no merge-format matrix loaded");
     CU(cudaStreamSynchronize(m->stream));
+    if (sliced(m)) {  // the chunks of host-array products are planned anew
+        m->pipe.K = 0;
+        m->pipe.rec.clear();
+    }
+    m->merge_only = true;
     m->l1 = variant | (m->P.colp16 ? 2 : 0);
     m->grid = merge_grid(m->cfg, m->num_tiles, m->sm_count, m->l1);
     m->pgrid = power_persistent_grid(kCfgF64, m->num_tiles, m->sm_count, m->l1);
     m->pgrid32 = power_persistent_grid(kCfgF32, m->num_tiles, m->sm_count, m->l1);
     m->pgridbf = power_persistent_grid(kCfgBF16, m->num_tiles, m->sm_count, m->l1);
+    return PWMGPU_OK;
+}
+
+int pwmgpu_layout(const pwmgpu_matrix* m, int precision, int32_t* layout) {
+    if (!m || !layout) return fail(PWMGPU_ERR_INVALID, "null handle or output");
+    if (precision != PWMGPU_PREC_F64 && precision != PWMGPU_PREC_F32)
+        return fail(PWMGPU_ERR_INVALID, "precision: F64 or F32");
+    if (!m->loaded) return fail(PWMGPU_ERR_STATE, "no matrix loaded");
+    const int fmt = fp64_format(m);
+    const bool low = precision == PWMGPU_PREC_F32;
+    if (fmt != PWMGPU_FMT_MERGE && !low)
+        *layout = fmt == PWMGPU_FMT_CSB ? PWMGPU_LAYOUT_CSB : PWMGPU_LAYOUT_COH;
+    else if (low && m->format != PWMGPU_FMT_MERGE)
+        return fail(PWMGPU_ERR_UNSUPPORTED, "FP32 SpMV runs on the merge format");
+    else if (sliced(m) &&
+             (!low || (m->low_format == PWMGPU_LOWFMT_AUTO && m->power_mode != PWMGPU_POWER_FUSED &&
+                       (m->diag.nslices ? m->diag.val32 : m->rows.val32))))
+        *layout = m->diag.nslices ? PWMGPU_LAYOUT_DIAGONALS : PWMGPU_LAYOUT_ROWS;
+    else if (low && m->low_format == PWMGPU_LOWFMT_AUTO && m->power_mode != PWMGPU_POWER_FUSED &&
+             m->sell.state == 1 && m->sell.val32)
+        *layout = PWMGPU_LAYOUT_SELL;
+    else
+        *layout = PWMGPU_LAYOUT_MERGE;
     return PWMGPU_OK;
 }
 

@@ -269,6 +269,13 @@ class CudaSparseMatrix:
         check(_lib.lib().pwmgpu_plan_info(self._h, C.byref(b), C.byref(g)), "pwmgpu_plan_info")
         return b.value, g.value
 
+    def layout(self, precision=PREC_F64):
+        """The layout products run on: "merge", "diagonals", "rows", "sell",
+        "csb" or "coh" (PREC_F32: of mv_device_f32, after its first call)."""
+        k = C.c_int32()
+        check(_lib.lib().pwmgpu_layout(self._h, int(precision), C.byref(k)), "pwmgpu_layout")
+        return _lib.LAYOUTS[k.value]
+
     def launch_variant(self):
         """The merge kernels' launch variant bits (pwmgpu_launch_variant)."""
         v = C.c_int32()
@@ -277,7 +284,8 @@ class CudaSparseMatrix:
 
     def set_launch_variant(self, variant):
         """Override the load-time tuner: 0 / 1 (shared-memory carveout), 4 / 5
-        (the same, x gathers around L1)."""
+        (the same, x gathers around L1).  A matrix on slices then runs on the
+        merge kernels until the next load."""
         check(_lib.lib().pwmgpu_set_launch_variant(self._h, int(variant)), "set_launch_variant")
 
     def tile_info(self):
