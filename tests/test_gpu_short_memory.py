@@ -1,0 +1,57 @@
+"""A load where device memory is short: what the handle cannot do without comes
+first, and slices beside the merge plan only from what its other calls do not
+need.  In a process of its own, with the rest of the memory held by torch."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import numpy as np, torch
+import thesis_spmv_gb300 as pwm
+from oracle import pyoracle as O
+M = pwm.CRSCuda(1)
+M.generatePoissonMatrix(8, 8, 1)
+def leave(gb):
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty(free - int(gb * (1 << 30)), dtype=torch.uint8, device="cuda")
+def check(m):
+    n = m * m
+    x = np.random.default_rng(1).random(n).reshape(m, m)
+    y = np.full(n, np.nan)
+    M.mv(x.reshape(-1), y)
+    p = np.zeros((m + 2, m + 2))
+    p[1:-1, 1:-1] = x
+    want = 4 * x - p[:-2, 1:-1] - p[2:, 1:-1] - p[1:-1, :-2] - p[1:-1, 2:]
+    assert np.all(np.abs(y.reshape(m, m) - want) <= 16 * 2.0 ** -53 * 8)
+"""
+
+
+def _run(body):
+    r = subprocess.run([sys.executable, "-c", HEAD + body + "\nprint('ok')"], capture_output=True, text=True, timeout=600,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout[-2000:] + r.stderr[-4000:]
+
+
+def test_a_load_that_fits_without_slices():
+    """4096^2 stencil: 1.0 GiB of CRS arrays and 1.0 of merge plan while it is
+    built, 0.7 of slices.  With 2.4 GiB left the slices do not fit beside them:
+    the load goes on without, and products and power steps have their memory."""
+    _run("""
+hog = leave(2.4)
+M.generatePoissonMatrix(4096, 4096, 1)
+assert M.layout() == "merge"
+check(4096)
+x, y = np.random.default_rng(2).random(4096 * 4096), np.zeros(4096 * 4096)
+M.powerIteration(x, y, 3)
+assert np.all(np.isfinite(y)) and abs(np.linalg.norm(y) - 1) < 1e-12
+del hog
+torch.cuda.empty_cache()
+M.generatePoissonMatrix(4096, 4096, 1)
+assert M.layout() == "diagonals"
+check(4096)
+""")

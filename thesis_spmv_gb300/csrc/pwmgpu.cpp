@@ -267,12 +267,30 @@ int build_col16(pwmgpu_matrix* m) {
     return PWMGPU_OK;
 }
 
+// The slices of a matrix beside its merge plan: diagonal ones where it fits
+// them, else sorted rows.  They take another 8 to 15 bytes per nonzero, so they
+// come after everything the handle cannot do without, and go back where less
+// is left than its other calls may ask for (CRS arrays or low-precision
+// values, vectors): the merge plan alone serves all of them.
+void build_slices(pwmgpu_matrix* m) {
+    const DevMatrix& M = m->M;
+    if (diag_build(m->diag, M.row_start, M.col, M.val, M.nor, M.nnz, m->sm_count, m->stream) != 0)
+        (void)rows_build(m->rows, M.row_start, M.col, M.val, M.nor, M.nnz, m->P.colp16 != nullptr, m->sm_count,
+                         m->stream);
+    const size_t spare = 12 * (size_t)M.nnz + 24 * (size_t)std::max(M.nor, M.noc);
+    if (!sliced(m) || spare < ((size_t)64 << 20)) return;  // (the question takes some 20 us)
+    size_t free_now = 0, total = 0;
+    if (cudaMemGetInfo(&free_now, &total) == cudaSuccess && free_now + dev_idle_bytes() >= spare) return;
+    (void)cudaGetLastError();
+    m->diag.release();
+    m->rows.release();
+}
+
 // The merge-path plan (and, with run_tuner, the load-time launch tuner).
 int build_merge(pwmgpu_matrix* m, bool run_tuner) {
-    // diagonal slices where the matrix fits them (no memory: the merge plan alone)
-    const bool diag =
-        diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count, m->stream) == 0;
-    if (diag && m->batched) {
+    // a serving loop's stencil: its diagonal slices alone
+    if (m->batched && diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count,
+                                 m->stream) == 0) {
         dfree(m->M.col);
         dfree(m->M.val);
         m->loaded = true;
@@ -298,13 +316,8 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
         CU(launch_mli_plan(m->M.row_start, m->M.col, m->M.val, P, m->sm_count, m->stream));
     }
     TRY(build_col16(m));
-    if (!diag && !m->batched)
-        (void)rows_build(m->rows, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->P.colp16 != nullptr,
-                         m->sm_count, m->stream);
     // fix-up descriptors; without them (no memory) the search-based fix-up runs
     (void)build_fix_runs(m->P, m->M.row_start, m->M.nor, m->sm_count, m->stream);
-    dfree(m->M.col);
-    dfree(m->M.val);
     m->l1 = m->P.colp16 ? 2 : 0;
     m->grid = merge_grid(m->cfg, m->num_tiles, m->sm_count, m->l1);
     m->fix_grid = fixup_grid(m->num_tiles, m->sm_count);
@@ -320,7 +333,10 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
     TRY(ensure_cap(m, &m->npart, &m->npart_cap,
                    (size_t)power_norm_parts(m->P, (int)std::min<long long>(((long long)m->num_tiles + 3) / 4,
                                                                            16LL * m->sm_count)) + 64));
+    if (!m->batched) build_slices(m);
     CU(cudaStreamSynchronize(m->stream));
+    dfree(m->M.col);
+    dfree(m->M.val);
     m->loaded = true;
     return run_tuner ? tune(m) : PWMGPU_OK;
 }
