@@ -55,3 +55,35 @@ M.generatePoissonMatrix(4096, 4096, 1)
 assert M.layout() == "diagonals"
 check(4096)
 """)
+
+
+def test_buffers_that_grow_where_memory_is_short():
+    """One handle, ever larger matrices: a buffer asks for twice the room of
+    the one it replaces, and is content with what it needs.  8192^2 rows after
+    6500^2: vectors of 0.5 GiB each, where twice the room were 0.63."""
+    _run("""
+M.generatePoissonMatrix(6500, 6500, 1)
+check(6500)
+M.generatePoissonMatrix(8, 8, 1)
+check(8)
+# 8192^2: 4.0 GiB of CRS arrays, 4.3 of plan while it is built
+hog = leave(8.9)
+M.generatePoissonMatrix(8192, 8192, 1)
+check(8192)
+""")
+
+
+def test_a_failed_load_leaves_the_memory_and_the_handle():
+    """Too little memory for the plan: an error, not a crash, and all that the
+    load had taken is back: the next, smaller one fits."""
+    _run("""
+hog = leave(1.5)
+for _ in range(3):
+    try:
+        M.generatePoissonMatrix(4096, 4096, 1)
+        raise SystemExit("the load should not have fitted")
+    except RuntimeError:
+        pass
+    M.generatePoissonMatrix(2048, 2048, 1)
+    check(2048)
+""")

@@ -99,6 +99,7 @@ cudaError_t dev_alloc(void** out, size_t bytes) {
         e = cudaMallocFromPoolAsync(out, bytes ? bytes : 1, p.pool, p.stream);
         if (e != cudaErrorMemoryAllocation) break;
         (void)cudaGetLastError();
+        (void)cudaStreamSynchronize(p.stream);  // (frees still under way hold their blocks)
         cudaMemPoolTrimTo(p.pool, 0);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(p.stream);

@@ -44,13 +44,26 @@ namespace {
 
 // Room for `need` elements in one of the handle's buffers.  The buffer it
 // replaces may still be in use on the stream: it goes back with the matrix
-// (twice the room each time bounds what waits there).
+// (twice the room each time bounds what waits there).  Where memory is short it
+// gets the room needed only, at last after the device has been waited for and
+// the buffers that wait have gone back.
 template <typename T>
 int ensure_cap(pwmgpu_matrix* m, T** p, size_t* cap, size_t need) {
     if (*cap >= need && *p) return PWMGPU_OK;
-    const size_t want = std::max(need, 2 * *cap);
+    size_t want = std::max(need, 2 * *cap);
     T* q = nullptr;
-    TRY(dalloc(&q, want));
+    int rc = dalloc(&q, want);
+    if (rc != PWMGPU_OK && want > need) rc = dalloc(&q, want = need);
+    if (rc != PWMGPU_OK) {
+        {
+            DevIdle idle(m->device);
+            for (void* o : m->outgrown) dev_free(o);
+            m->outgrown.clear();
+            dfree(*p);
+            *cap = 0;
+        }
+        TRY(dalloc(&q, need));
+    }
     if (*p) m->outgrown.push_back(*p);
     *p = q;
     *cap = want;
