@@ -61,7 +61,10 @@ typedef struct pwmgpu_matrix pwmgpu_matrix;
 /* Message of the calling thread's last failing call ("" if none). */
 const char* pwmgpu_last_error(void);
 
-/* Device facts for the current device. */
+/* Device facts for the current device.  free_bytes counts what this library can
+ * still allocate: the device's free memory and what its own pool holds idle (up
+ * to 1/64 of the device while handles live, 1/1024 after; other allocators do
+ * not see the pool's part). */
 int pwmgpu_device_info(int* sm_count, size_t* free_bytes, size_t* total_bytes);
 
 /* Replaces the reference constructors `CRS_Merge(int threads)`,

@@ -110,13 +110,44 @@ A = pwm.CRSCuda(1); A.generatePoissonMatrix(2048, 2048, 1)
 B = pwm.CRSCuda(1); B.generatePoissonMatrix(64, 48, 1)
 assert torch.cuda.mem_get_info()[0] < free0 - (200 << 20)
 del A, B
-assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20), (free0, torch.cuda.mem_get_info())
+free1, total = torch.cuda.mem_get_info()
+assert free1 >= free0 - total // 1024 - (64 << 20), (free0, free1)
 print("ok")
 """
 
 
 def test_pool_goes_back_with_the_last_handle():
-    """(in a process of its own: other tests' handles would keep the pool)"""
+    """All but 1/1024 of the device's memory, which stays for the next handle.
+    (In a process of its own: other tests' handles would keep the pool.)"""
     r = subprocess.run([sys.executable, "-c", POOL], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+LONE = """
+import time, torch, thesis_spmv_gb300 as pwm
+torch.zeros(1, device="cuda")
+def cycle():
+    best = 1e9
+    for _ in range(12):
+        t = time.perf_counter()
+        M = pwm.CRSCuda(1)
+        M.generatePoissonMatrix(64, 48, 1)
+        del M
+        best = min(best, time.perf_counter() - t)
+    return best
+lone = cycle()
+K = pwm.CRSCuda(1)
+beside = cycle()
+assert lone <= 2 * beside, (lone, beside)
+print("ok")
+"""
+
+
+def test_one_small_handle_after_another():
+    """Made, loaded and dropped with no other handle alive, a small handle costs
+    what it costs beside one (it mapped and unmapped its memory each time: 0.8 ms
+    and 0.25)."""
+    r = subprocess.run([sys.executable, "-c", LONE], capture_output=True, text=True, timeout=300,
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr

@@ -74,12 +74,27 @@ struct SliceWalk {
 };
 
 // Slots per slice (ptr[c + 1], scanned afterwards), their sum in 64 bits, and
-// flag = 1 once a slice exceeds kDiagMaxSlots (the rest then stops early).
+// flag = 1 once a slice exceeds kDiagMaxSlots or the sum exceeds `most` (the
+// rest then stops early).  A CTA adds its slots to the sum 512 at a time -- an
+// addition per warp takes half a millisecond on 4 M rows -- and 64 at a time
+// where there are few, so that a small matrix stops in time (1024 irregular
+// rows: 25 us sooner).
 __global__ void __launch_bounds__(256) k_diag_count(const int32_t* __restrict__ row_start,
                                                     const int32_t* __restrict__ col, int nor, int nslices,
-                                                    int32_t* __restrict__ ptr, unsigned long long* total, int* flag) {
+                                                    unsigned long long most, int32_t* __restrict__ ptr,
+                                                    unsigned long long* total, int* flag) {
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    unsigned long long sum = 0;
+    const int step = nslices <= 4096 ? 6 : 9;
+    __shared__ unsigned slots;  // of the CTA's slices
+    unsigned sum = 0;           // of the warp's
+    if (threadIdx.x == 0) slots = 0u;
+    __syncthreads();
+    // n more slots; whether the sum of all is known to exceed `most`
+    auto add = [&](unsigned n) {
+        const unsigned before = atomicAdd(&slots, n);
+        const unsigned long long whole = ((before + n) >> step) - (before >> step);
+        return whole && atomicAdd(total, whole << step) + (whole << step) > most;
+    };
     for (int c = blockIdx.x * wpb + (threadIdx.x >> 5); c < nslices; c += gridDim.x * wpb) {
         if (__any_sync(0xffffffffu, *(volatile int*)flag)) break;
         SliceWalk w(row_start, col, nor, c, lane);
@@ -91,14 +106,21 @@ __global__ void __launch_bounds__(256) k_diag_count(const int32_t* __restrict__ 
                     ++w.cur[r];
                     w.load(col, r);
                 }
+            if ((++sum & 63) == 0) {
+                const bool over = lane == 0 && add(64u);
+                if (over) *(volatile int*)flag = 1;
+                if (__any_sync(0xffffffffu, over)) break;
+            }
         }
         if (lane == 0) {
             ptr[c + 1] = n;
             if (n > kDiagMaxSlots) *(volatile int*)flag = 1;
         }
-        sum += (unsigned long long)n;
     }
-    if (lane == 0 && sum) atomicAdd(total, sum);
+    if (lane == 0) (void)add(sum & 63);
+    __syncthreads();
+    const unsigned left = slots & ((1u << step) - 1u);
+    if (threadIdx.x == 0 && left) atomicAdd(total, (unsigned long long)left);
 }
 
 // The slots' offsets, masks and FP64 values, and the slices' records.
@@ -334,67 +356,78 @@ void DiagPlan::release() {
     *this = DiagPlan();
 }
 
-int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
-               int sm_count, cudaStream_t st) {
-    D.release();
+// One allocation of scratch (DiagFound, slots per slice, the scan's), one of
+// the plan: on a small matrix the allocations and waits are the build's cost.
+namespace {
+// Stored elements within 1.25 of the nonzeros: at that line the layout
+// streams 10.1 bytes per nonzero, as much as the merge layout at its
+// best (10, plus a fix-up kernel).  (128 slots more: a few slices,
+// where either is one launch's latency.)
+unsigned long long most_slots(long long nnz) {
+    return (unsigned long long)((1.25 * (double)nnz + 128.0 * kDiagRows) / kDiagRows);
+}
+int* slot_ptr(const DiagBuild& B) { return reinterpret_cast<int32_t*>(B.tmp + sizeof(DiagFound)); }
+int fill_blocks(int nslices, int sm_count) {
+    return (int)std::min<long long>(((long long)nslices + 7) / 8, 32LL * sm_count);
+}
+}  // namespace
+
+int diag_count(DiagBuild& B, const int32_t* row_start, const int32_t* col, int nor, long long nnz, int sm_count,
+               Scratch& scratch, DiagFound* found, cudaStream_t st) {
+    B = DiagBuild();
     if (nor <= 0 || nnz <= 0) return 1;
     const int ns = (nor + kDiagRows - 1) / kDiagRows;
-    const int blocks = (int)std::min<long long>(((long long)ns + 7) / 8, 32LL * sm_count);
-    struct Head {
-        unsigned long long total;
-        int flag, pad;
-    } h{0, 0, 0};
-    // one allocation of scratch (total and flag, slots per slice, the scan's),
-    // one of the plan: on a small matrix the allocations are the build's cost
-    const size_t ptr_at = sizeof(Head), scan_at = ptr_at + sizeof(int32_t) * ((size_t)ns + 1);
-    unsigned char* tmp = nullptr;
-    int rc = 2;
-    do {
-        if (dev_alloc((void**)&tmp, scan_at + sizeof(int32_t) * (size_t)scan_scratch_elems(ns)) != cudaSuccess) break;
-        Head* dh = reinterpret_cast<Head*>(tmp);
-        int32_t* ptr = reinterpret_cast<int32_t*>(tmp + ptr_at);
-        if (cudaMemsetAsync(tmp, 0, ptr_at + sizeof(int32_t), st) != cudaSuccess) break;
-        k_diag_count<<<blocks, 256, 0, st>>>(row_start, col, nor, ns, ptr, &dh->total, &dh->flag);
-        if (cudaMemcpyAsync(&h, dh, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess) break;
-        if (cudaStreamSynchronize(st) != cudaSuccess) break;
-        // Stored elements within 1.25 of the nonzeros: at that line the layout
-        // streams 10.1 bytes per nonzero, as much as the merge layout at its
-        // best (10, plus a fix-up kernel).  (128 slots more: a few slices,
-        // where either is one launch's latency.)
-        if (h.flag || (double)h.total * kDiagRows > 1.25 * (double)nnz + 128.0 * kDiagRows) {
-            rc = 1;
-            break;
-        }
-        const size_t slots = (size_t)h.total, elems = slots * kDiagRows;
-        auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
-        const size_t vb = up(sizeof(double) * (elems + 1)), rb = up(sizeof(int2) * (size_t)ns),
-                     mb = up(sizeof(SlotMask) * (slots + 1)), ob = up(sizeof(int32_t) * (slots + 1)),
-                     nb = sizeof(double) * kDiagMaxCtas * (size_t)sm_count;
-        if (launch_inclusive_scan(ptr + 1, ns, reinterpret_cast<int32_t*>(tmp + scan_at), st) != cudaSuccess) break;
-        if (dev_alloc(&D.mem, vb + rb + mb + ob + nb) != cudaSuccess) {
-            D.mem = nullptr;
-            break;
-        }
+    const size_t heads = sizeof(DiagFound) + sizeof(int32_t);
+    cudaError_t e = scratch.alloc(&B.tmp, heads + sizeof(int32_t) * ((size_t)ns + (size_t)scan_scratch_elems(ns)));
+    if (e == cudaSuccess) e = cudaMemsetAsync(B.tmp, 0, heads, st);
+    if (e == cudaSuccess) {
+        DiagFound* d = reinterpret_cast<DiagFound*>(B.tmp);
+        k_diag_count<<<fill_blocks(ns, sm_count), 256, 0, st>>>(row_start, col, nor, ns, most_slots(nnz), slot_ptr(B),
+                                                                &d->total, &d->flag);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(found, B.tmp, sizeof *found, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 2;
+    }
+    B.nslices = ns;
+    return 0;
+}
+
+int diag_fill(DiagPlan& D, const DiagBuild& B, const DiagFound& found, const int32_t* row_start, const int32_t* col,
+              const double* val, int nor, long long nnz, int sm_count, cudaStream_t st) {
+    D.release();
+    if (found.flag || found.total > most_slots(nnz)) return 1;
+    const int ns = B.nslices;
+    const size_t slots = (size_t)found.total, elems = slots * kDiagRows;
+    auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    const size_t vb = up(sizeof(double) * (elems + 1)), rb = up(sizeof(int2) * (size_t)ns),
+                 mb = up(sizeof(SlotMask) * (slots + 1)), ob = up(sizeof(int32_t) * (slots + 1)),
+                 nb = sizeof(double) * kDiagMaxCtas * (size_t)sm_count;
+    int32_t* ptr = slot_ptr(B);
+    cudaError_t e = dev_alloc(&D.mem, vb + rb + mb + ob + nb);
+    if (e == cudaSuccess) e = launch_inclusive_scan(ptr + 1, ns, ptr + 1 + ns, st);
+    if (e == cudaSuccess) {
         unsigned char* p = static_cast<unsigned char*>(D.mem);
         D.val64 = reinterpret_cast<double*>(p);
         D.rec = reinterpret_cast<int2*>(p + vb);
         D.masks = p + vb + rb;
         D.offs = reinterpret_cast<int32_t*>(p + vb + rb + mb);
         D.npart = reinterpret_cast<double*>(p + vb + rb + mb + ob);
-        k_diag_fill<<<blocks, 256, 0, st>>>(row_start, col, val, nor, ns, ptr, D.rec, D.offs, (SlotMask*)D.masks,
-                                            D.val64);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) break;
-        D.nslices = ns;
-        D.elems = (long long)elems;
-        rc = 0;
-    } while (0);
-    (void)cudaStreamSynchronize(st);
-    dev_free(tmp);
-    if (rc) {
-        (void)cudaGetLastError();
-        D.release();
+        k_diag_fill<<<fill_blocks(ns, sm_count), 256, 0, st>>>(row_start, col, val, nor, ns, ptr, D.rec, D.offs,
+                                                               (SlotMask*)D.masks, D.val64);
+        e = cudaGetLastError();
     }
-    return rc;
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (D.mem) (void)cudaStreamSynchronize(st);
+        D.release();
+        return 2;
+    }
+    D.nslices = ns;
+    D.elems = (long long)elems;
+    return 0;
 }
 
 int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st) {

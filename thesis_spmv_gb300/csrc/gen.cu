@@ -253,6 +253,7 @@ cudaError_t launch_inclusive_scan(int32_t* a, long long n, int32_t* scratch, cud
     if (n <= 0) return cudaSuccess;
     const long long nt = (n + kScanTile - 1) / kScanTile;
     k_scan_tiles<<<(unsigned)nt, kScanThreads, 0, st>>>(a, n, scratch);
+    if (nt == 1) return cudaGetLastError();
     k_scan_sums<<<1, kScanThreads, 0, st>>>(scratch, (int)nt);
     k_scan_add<<<(unsigned)nt, kScanThreads, 0, st>>>(a, n, scratch);
     return cudaGetLastError();

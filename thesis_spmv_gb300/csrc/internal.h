@@ -66,7 +66,38 @@ private:
 };
 // Bytes the current device's pool holds without using them.
 size_t dev_idle_bytes();
-// A pinned host block of 128 bytes.
+// Device blocks of a build whose kernels may still be under way: they go back
+// after a wait for the stream, one for all of them.
+class Scratch {
+public:
+    explicit Scratch(cudaStream_t st) : st_(st) {}
+    ~Scratch() { release(); }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    template <typename T>
+    cudaError_t alloc(T** p, size_t bytes) {
+        *p = nullptr;
+        if (n_ == kMost) return cudaErrorMemoryAllocation;
+        const cudaError_t e = dev_alloc((void**)p, bytes);
+        if (e == cudaSuccess) blocks_[n_++] = *p;
+        else *p = nullptr;
+        return e;
+    }
+    void release() {
+        if (n_ == 0) return;
+        (void)cudaStreamSynchronize(st_);
+        while (n_ > 0) dev_free(blocks_[--n_]);
+    }
+
+private:
+    static constexpr int kMost = 8;
+    void* blocks_[kMost];
+    int n_ = 0;
+    cudaStream_t st_;
+};
+// A pinned host block: what a handle reads back from the device (a copy into
+// pageable memory would wait for the stream by itself, some 8 us each).
+constexpr size_t kPinnedBlock = 1024;
 cudaError_t pinned_alloc(void** out);
 void pinned_free(void* p);
 
@@ -132,12 +163,25 @@ struct DiagPlan {
     double* npart = nullptr;     // per-CTA shares of ||y||^2
     void release();
 };
-// 0 = built, 1 = the matrix does not fit (D stays empty), 2 = a CUDA error or
-// no memory (D stays empty).
-int diag_build(DiagPlan& D, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
-               int sm_count, cudaStream_t st);
+// The slices of a CRS matrix, in two steps with a wait for the stream between
+// them and, before the CRS arrays or the scratch go, after them: the kernels of
+// diag_count leave what they find in `found`, pinned host memory.  0 = on the
+// way, 1 = the matrix does not fit (D stays empty), 2 = a CUDA error or no
+// memory (D stays empty).
+struct DiagFound {
+    unsigned long long total;  // slots
+    int flag, pad;             // flag: a slice has more than it may
+};
+struct DiagBuild {
+    unsigned char* tmp = nullptr;
+    int nslices = 0;
+};
+int diag_count(DiagBuild& B, const int32_t* row_start, const int32_t* col, int nor, long long nnz, int sm_count,
+               Scratch& scratch, DiagFound* found, cudaStream_t st);
+int diag_fill(DiagPlan& D, const DiagBuild& B, const DiagFound& found, const int32_t* row_start, const int32_t* col,
+              const double* val, int nor, long long nnz, int sm_count, cudaStream_t st);
 // The values in FP32 / BF16, made on first use and complete on return (the
-// stream is synchronised: not inside a capture).  0, or 2 as diag_build.
+// stream is synchronised: not inside a capture).  0, or 2 as diag_fill.
 int diag_low_values(DiagPlan& D, bool bf16, int sm_count, cudaStream_t st);
 // One pass over slices [c0, c1) (c1 < 0: all).  mode kModeSpmv: y = A x;
 // kModePower: y = 2^e A x and *nsq_out = ||y||^2 (when given; counter zero
@@ -177,10 +221,11 @@ struct RowsPlan {
     double* npart = nullptr;     // per-CTA shares of ||y||^2
     void release();
 };
-// 0 = built, 1 = the matrix does not fit, 2 = a CUDA error or no memory (R
-// stays empty).
+// pinned: kPinnedBlock bytes.  0 = on the way (the CRS arrays and the scratch
+// are in use until the stream has been waited for), 1 = the matrix does not fit, 2 = a CUDA error or no
+// memory (R stays empty).
 int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
-               bool narrow, int sm_count, cudaStream_t st);
+               bool narrow, int sm_count, Scratch& keep, void* pinned, cudaStream_t st);
 // As diag_low_values.
 int rows_low_values(RowsPlan& R, bool bf16, int sm_count, cudaStream_t st);
 // Pipelined host-array SpMV: out[w] = the largest column of windows 0 .. w.
@@ -230,9 +275,13 @@ cudaError_t launch_power_norm_f32(const float* y, const float* x, int n, double*
 cudaError_t launch_solve_result(bool f32, const void* in, const void* out, int n, const double* nsq_k,
                                 const double* nd, double* nsq_next, double* result, double* partials,
                                 unsigned int* counter, int grid, cudaStream_t st);
-// fix-up run descriptors of a plan (P.runs, P.run_pre, P.nruns; scratch: 2 *
-// (nsub + 1) ints and nsub int4) and the fix-up over descriptors [k0, k1)
-int build_fix_runs(MliPlan& P, const int32_t* row_start, int nor, int sm_count, cudaStream_t st);
+// fix-up run descriptors of a plan (P.runs, P.run_pre, P.nruns), counted and
+// filled with a wait for the stream between (`found`: pinned) and before the
+// scratch goes; 0, or 1 where they cannot be made
+int fix_runs_count(MliPlan& P, const int32_t* row_start, int nor, int4** desc, Scratch& scratch, int* found,
+                   cudaStream_t st);
+int fix_runs_fill(MliPlan& P, const int4* desc, int found, cudaStream_t st);
+// and the fix-up over descriptors [k0, k1)
 cudaError_t launch_fix_runs_f64(int mode, const MliPlan& P, int k0, int k1, double* y, const double* carries,
                                 const double* nsq_in, cudaStream_t st);
 cudaError_t launch_fix_runs_f32(int mode, const MliPlan& P, int k0, int k1, float* y, const float* carries,

@@ -1338,49 +1338,54 @@ cudaError_t launch_solve_result(bool f32, const void* in, const void* out, int n
     return cudaGetLastError();
 }
 
-int build_fix_runs(MliPlan& P, const int32_t* row_start, int nor, int sm_count, cudaStream_t st) {
-    (void)sm_count;
+int fix_runs_count(MliPlan& P, const int32_t* row_start, int nor, int4** desc, Scratch& scratch, int* found,
+                   cudaStream_t st) {
     P.nruns = 0;
-    if (P.nsub <= 0) return 0;
-    int* scan_scratch = nullptr;
-    int4* desc = nullptr;
-    int rc = 0;
-    const int nb = (P.nsub + 255) / 256;
-    do {
-        if (dev_alloc((void**)&desc, sizeof(int4) * (size_t)P.nsub) != cudaSuccess ||
-            dev_alloc((void**)&scan_scratch, sizeof(int) * (size_t)scan_scratch_elems(P.nsub + 1)) != cudaSuccess ||
-            dev_alloc((void**)&P.run_pre, sizeof(int) * ((size_t)P.nsub + 1)) != cudaSuccess) {
-            rc = 1;
-            break;
-        }
-        // run_pre[0] = 0, run_pre[t + 1] = flag[t]; the inclusive scan of
-        // run_pre + 1 makes run_pre[t] the runs that start before t
-        if (cudaMemsetAsync(P.run_pre, 0, sizeof(int), st) != cudaSuccess) { rc = 1; break; }
-        k_run_flags<<<nb, 256, 0, st>>>(row_start, P.subc, P.nsub, nor, P.run_pre + 1, desc);
-        if (launch_inclusive_scan(P.run_pre + 1, P.nsub, scan_scratch, st) != cudaSuccess) { rc = 1; break; }
-        int total = 0;
-        if (cudaMemcpyAsync(&total, P.run_pre + P.nsub, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
-            rc = 1;
-            break;
-        }
-        P.nruns = total;
-        if (dev_alloc((void**)&P.runs, sizeof(int4) * (size_t)(total > 0 ? total : 1)) != cudaSuccess) { rc = 1; break; }
-        if (total > 0) k_run_compact<<<nb, 256, 0, st>>>(P.run_pre, desc, P.nsub, P.runs);
-        if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = 1;
-    } while (0);
-    (void)cudaStreamSynchronize(st);
-    dev_free(desc);
-    dev_free(scan_scratch);
-    if (rc) {
+    *desc = nullptr;
+    if (P.nsub <= 0) return 1;
+    int* scan = nullptr;
+    // desc: 16-byte records, then the scan's words
+    const size_t db = sizeof(int4) * (size_t)P.nsub;
+    if (scratch.alloc(desc, db + sizeof(int) * (size_t)scan_scratch_elems(P.nsub)) != cudaSuccess ||
+        dev_alloc((void**)&P.run_pre, sizeof(int) * ((size_t)P.nsub + 1)) != cudaSuccess) {
         (void)cudaGetLastError();
-        dev_free(P.runs);
-        dev_free(P.run_pre);
-        P.runs = nullptr;
         P.run_pre = nullptr;
-        P.nruns = 0;
+        return 1;
     }
-    return rc;
+    scan = reinterpret_cast<int*>(*desc + P.nsub);
+    // run_pre[0] = 0, run_pre[t + 1] = flag[t]; the inclusive scan of
+    // run_pre + 1 makes run_pre[t] the runs that start before t
+    cudaError_t e = cudaMemsetAsync(P.run_pre, 0, sizeof(int), st);
+    if (e == cudaSuccess) {
+        k_run_flags<<<(P.nsub + 255) / 256, 256, 0, st>>>(row_start, P.subc, P.nsub, nor, P.run_pre + 1, *desc);
+        e = launch_inclusive_scan(P.run_pre + 1, P.nsub, scan, st);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(found, P.run_pre + P.nsub, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) return 0;
+    (void)cudaGetLastError();
+    (void)cudaStreamSynchronize(st);
+    dev_free(P.run_pre);
+    P.run_pre = nullptr;
+    return 1;
+}
+
+int fix_runs_fill(MliPlan& P, const int4* desc, int found, cudaStream_t st) {
+    cudaError_t e = dev_alloc((void**)&P.runs, sizeof(int4) * (size_t)(found > 0 ? found : 1));
+    if (e == cudaSuccess && found > 0) {
+        k_run_compact<<<(P.nsub + 255) / 256, 256, 0, st>>>(P.run_pre, desc, P.nsub, P.runs);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+        P.nruns = found;
+        return 0;
+    }
+    (void)cudaGetLastError();
+    (void)cudaStreamSynchronize(st);
+    dev_free(P.runs);
+    dev_free(P.run_pre);
+    P.runs = nullptr;
+    P.run_pre = nullptr;
+    return 1;
 }
 
 template <typename XT, typename AT>

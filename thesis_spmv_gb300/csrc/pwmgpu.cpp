@@ -245,70 +245,94 @@ int tune(pwmgpu_matrix* m) {
 
 // 16-bit columns for the merge kernels when every sub-tile's columns span
 // less than 2^16 (then the SpMV streams 10 bytes per FP64 nonzero instead of
-// 12).  Skipped, not an error, when the span is wider or the extra array does
-// not fit.
-int build_col16(pwmgpu_matrix* m) {
+// 12): whether they do, then the columns.  Skipped, not an error, when the span
+// is wider or the extra array does not fit.
+int col16_count(pwmgpu_matrix* m, int** cbase, Scratch& scratch, int* wide) {
     MliPlan& P = m->P;
+    *wide = 1;
+    *cbase = nullptr;
     if (P.nsub == 0 || m->M.nnz == 0) return PWMGPU_OK;
-    int* cbase = nullptr;
-    int* flag = nullptr;
-    TRY(dalloc(&cbase, (size_t)P.nsub));
-    int rc = dalloc(&flag, 1);
-    int wide = 1;
-    cudaError_t e = cudaSuccess;
-    if (rc == PWMGPU_OK) {
-        e = cudaMemsetAsync(flag, 0, sizeof(int), m->stream);
-        if (e == cudaSuccess) e = launch_mli_colspan(P, cbase, flag, m->sm_count, m->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, m->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    }
-    if (rc == PWMGPU_OK && e == cudaSuccess && !wide) {
-        const size_t elems = (size_t)mli_storage_elems(m->M.nnz, P.nsub);
-        if (dev_alloc((void**)&P.colp16, elems * sizeof(uint16_t)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            P.colp16 = nullptr;
-        } else {
-            e = cudaMemsetAsync(P.colp16, 0, elems * sizeof(uint16_t), m->stream);
-            if (e == cudaSuccess) e = launch_mli_col16(P, cbase, m->sm_count, m->stream);
-        }
-    }
-    (void)cudaStreamSynchronize(m->stream);
-    dfree(cbase);
-    dfree(flag);
-    if (rc != PWMGPU_OK) return rc;
-    if (e != cudaSuccess) return fail(PWMGPU_ERR_CUDA, "16-bit column plan: %s", cudaGetErrorString(e));
+    if (scratch.alloc(cbase, sizeof(int) * ((size_t)P.nsub + 1)) != cudaSuccess)
+        return fail(PWMGPU_ERR_NOMEM, "no memory for the plan of 16-bit columns");
+    int* flag = *cbase + P.nsub;
+    CU(cudaMemsetAsync(flag, 0, sizeof(int), m->stream));
+    CU(launch_mli_colspan(P, *cbase, flag, m->sm_count, m->stream));
+    CU(cudaMemcpyAsync(wide, flag, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     return PWMGPU_OK;
 }
+
+int col16_fill(pwmgpu_matrix* m, const int* cbase) {
+    MliPlan& P = m->P;
+    const size_t elems = (size_t)mli_storage_elems(m->M.nnz, P.nsub);
+    if (dev_alloc((void**)&P.colp16, elems * sizeof(uint16_t)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        P.colp16 = nullptr;
+        return PWMGPU_OK;
+    }
+    CU(cudaMemsetAsync(P.colp16, 0, elems * sizeof(uint16_t), m->stream));
+    CU(launch_mli_col16(P, cbase, m->sm_count, m->stream));
+    return PWMGPU_OK;
+}
+
+// What a load's counting kernels find, in the handle's pinned block.
+struct PlanFound {
+    DiagFound diag;
+    int wide, runs;
+};
+static_assert(sizeof(PlanFound) <= kPinnedBlock, "the pinned block");
 
 // The slices of a matrix beside its merge plan: diagonal ones where it fits
 // them, else sorted rows.  They take another 8 to 15 bytes per nonzero, so they
 // come after everything the handle cannot do without, and go back where less
-// is left than its other calls may ask for (CRS arrays or low-precision
-// values, vectors): the merge plan alone serves all of them.
-void build_slices(pwmgpu_matrix* m) {
+// is left than its other calls may ask for (CRS arrays, as many bytes as those
+// of the load that go back now, or low-precision values; vectors): the merge
+// plan alone serves all of them.
+void build_slices(pwmgpu_matrix* m, const DiagBuild& B, const DiagFound& found, Scratch& scratch) {
     const DevMatrix& M = m->M;
-    if (diag_build(m->diag, M.row_start, M.col, M.val, M.nor, M.nnz, m->sm_count, m->stream) != 0)
+    if (!B.nslices ||
+        diag_fill(m->diag, B, found, M.row_start, M.col, M.val, M.nor, M.nnz, m->sm_count, m->stream) != 0)
         (void)rows_build(m->rows, M.row_start, M.col, M.val, M.nor, M.nnz, m->P.colp16 != nullptr, m->sm_count,
-                         m->stream);
-    const size_t spare = 12 * (size_t)M.nnz + 24 * (size_t)std::max(M.nor, M.noc);
-    if (!sliced(m) || spare < ((size_t)64 << 20)) return;  // (the question takes some 20 us)
+                         scratch, m->hres, m->stream);
+    const size_t spare = 24 * (size_t)std::max(M.nor, M.noc);
+    if (!sliced(m) || spare + 12 * (size_t)M.nnz < ((size_t)64 << 20)) return;  // (the question takes some 20 us)
     size_t free_now = 0, total = 0;
     if (cudaMemGetInfo(&free_now, &total) == cudaSuccess && free_now + dev_idle_bytes() >= spare) return;
     (void)cudaGetLastError();
+    (void)cudaStreamSynchronize(m->stream);
     m->diag.release();
     m->rows.release();
 }
 
-// The merge-path plan (and, with run_tuner, the load-time launch tuner).
+// A serving loop's stencil: its diagonal slices alone.
+bool build_diag_only(pwmgpu_matrix* m) {
+    const DevMatrix& M = m->M;
+    auto* found = reinterpret_cast<DiagFound*>(m->hres);
+    Scratch scratch(m->stream);
+    DiagBuild B;
+    return diag_count(B, M.row_start, M.col, M.nor, M.nnz, m->sm_count, scratch, found, m->stream) == 0 &&
+           cudaStreamSynchronize(m->stream) == cudaSuccess &&
+           diag_fill(m->diag, B, *found, M.row_start, M.col, M.val, M.nor, M.nnz, m->sm_count, m->stream) == 0;
+}
+
+// The merge-path plan and the slices beside it (and, with run_tuner, the
+// load-time launch tuner).  The kernels that count -- slots, the columns'
+// span, fix-up runs -- run one after the other, then one wait, then the ones
+// that fill what the counts sized, then another: on a small matrix the waits are
+// most of the load.
 int build_merge(pwmgpu_matrix* m, bool run_tuner) {
-    // a serving loop's stencil: its diagonal slices alone
-    if (m->batched && diag_build(m->diag, m->M.row_start, m->M.col, m->M.val, m->M.nor, m->M.nnz, m->sm_count,
-                                 m->stream) == 0) {
+    if (m->batched && build_diag_only(m)) {
+        CU(cudaStreamSynchronize(m->stream));
         dfree(m->M.col);
         dfree(m->M.val);
         m->loaded = true;
         return PWMGPU_OK;
     }
+    auto* found = reinterpret_cast<PlanFound*>(m->hres);
+    Scratch scratch(m->stream);
+    DiagBuild slots;
+    if (!m->batched)
+        (void)diag_count(slots, m->M.row_start, m->M.col, m->M.nor, m->M.nnz, m->sm_count, scratch, &found->diag,
+                         m->stream);
     const long long total = (long long)m->M.nor + m->M.nnz;
     const MergeGeom g = merge_geometry(m->cfg);
     m->tm = g.wm;
@@ -328,9 +352,14 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
         CU(launch_merge_partition(m->M.row_start, m->M.nor, m->M.nnz, m->tm, P.nsub, P.subc, m->stream));
         CU(launch_mli_plan(m->M.row_start, m->M.col, m->M.val, P, m->sm_count, m->stream));
     }
-    TRY(build_col16(m));
+    int* cbase = nullptr;
+    int4* desc = nullptr;
+    TRY(col16_count(m, &cbase, scratch, &found->wide));
+    const bool runs = fix_runs_count(P, m->M.row_start, m->M.nor, &desc, scratch, &found->runs, m->stream) == 0;
+    CU(cudaStreamSynchronize(m->stream));
+    if (!found->wide) TRY(col16_fill(m, cbase));
     // fix-up descriptors; without them (no memory) the search-based fix-up runs
-    (void)build_fix_runs(m->P, m->M.row_start, m->M.nor, m->sm_count, m->stream);
+    if (runs) (void)fix_runs_fill(P, desc, found->runs, m->stream);
     m->l1 = m->P.colp16 ? 2 : 0;
     m->grid = merge_grid(m->cfg, m->num_tiles, m->sm_count, m->l1);
     m->fix_grid = fixup_grid(m->num_tiles, m->sm_count);
@@ -346,7 +375,7 @@ int build_merge(pwmgpu_matrix* m, bool run_tuner) {
     TRY(ensure_cap(m, &m->npart, &m->npart_cap,
                    (size_t)power_norm_parts(m->P, (int)std::min<long long>(((long long)m->num_tiles + 3) / 4,
                                                                            16LL * m->sm_count)) + 64));
-    if (!m->batched) build_slices(m);
+    if (!m->batched) build_slices(m, slots, found->diag, scratch);
     CU(cudaStreamSynchronize(m->stream));
     dfree(m->M.col);
     dfree(m->M.val);
@@ -1359,7 +1388,8 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
         if ((rc = dalloc(&scan_scratch, (size_t)scan_scratch_elems(nor))) != PWMGPU_OK) break;
         if ((rc = dalloc(&pos, (size_t)nnz)) != PWMGPU_OK) break;
         if ((rc = dalloc(&dflags, 1)) != PWMGPU_OK) break;
-        TripletScan flags{~0ull, 0u, 0u, 0, 0};
+        auto& flags = *reinterpret_cast<TripletScan*>(m->hres);
+        flags = TripletScan{~0ull, 0u, 0u, 0, 0};
         cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nor + 1), m->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dflags, &flags, sizeof flags, cudaMemcpyHostToDevice, m->stream);
         if (e == cudaSuccess)
@@ -1382,7 +1412,7 @@ int load_triplets_dev(pwmgpu_matrix* m, int32_t nor, int32_t noc, int32_t nnz, c
         // rows sorted in shared memory or all entries by radix
         bool by_rows = flags.unsorted_rc && triplet_rows_fit(flags.longest, nullptr, nnz);
         if (flags.unsorted_rc && !by_rows) {
-            TripletWork work{};
+            auto& work = *reinterpret_cast<TripletWork*>(&flags + 1);
             if ((rc = dalloc(&dwork, 1)) != PWMGPU_OK) break;
             e = launch_triplet_work(cnt + 1, nor, dwork, m->sm_count, m->stream);
             if (e == cudaSuccess) e = cudaMemcpyAsync(&work, dwork, sizeof work, cudaMemcpyDeviceToHost, m->stream);

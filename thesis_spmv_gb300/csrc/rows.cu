@@ -52,11 +52,11 @@ struct RowsCut {
 };
 constexpr int kRowsLate = 512;  // elements of a row that may start last
 // Rows of each window by class (0: a warp, 1: four lanes, 2: a lane each), the
-// longest row, and the units of all items (summed later).
-// And where each (window, class) starts, in items and in sorted rows.
+// first item of each (window, class), the longest row, and the units of all
+// items.
 struct RowsHead {
     int rows[3 * kRowsWindows];
-    int item[3 * kRowsWindows + 1], row[3 * kRowsWindows];
+    int item[3 * kRowsWindows + 1];
     int longest;
     unsigned long long units;
 };
@@ -92,29 +92,32 @@ __global__ void __launch_bounds__(256) k_rows_keys(const int32_t* __restrict__ r
         if (cnt[i]) atomicAdd(&head->rows[i], cnt[i]);
 }
 
-__global__ void k_rows_segs(RowsHead* h) {
-    int items = 0, rows = 0;
-    for (int k = 0; k < 3 * kRowsWindows; ++k) {
-        const int n = h->rows[k], per = 32 >> class_shift(k % 3);
-        h->item[k] = items;
-        h->row[k] = rows;
-        items += (n + per - 1) / per;
-        rows += n;
-    }
-    h->item[3 * kRowsWindows] = items;
-}
-
-// Items: their rows, and the units of each (off[i + 1], zero before and
-// scanned afterwards).
+// Items: where each (window, class) starts among them, their rows, and the
+// units of each (off[i + 1], zero before and scanned afterwards).
 __global__ void __launch_bounds__(256) k_rows_items(const int32_t* __restrict__ row_start,
                                                     const int32_t* __restrict__ perm, RowsHead* head,
                                                     int4* __restrict__ rec, int32_t* __restrict__ off) {
-    __shared__ RowsHead h;
-    for (int i = threadIdx.x; i < (int)(sizeof h / 4); i += blockDim.x)
-        reinterpret_cast<int*>(&h)[i] = reinterpret_cast<const int*>(head)[i];
+    constexpr int classes = 3 * kRowsWindows;
+    __shared__ struct {
+        int rows[classes], item[classes + 1], row[classes];
+    } h;
+    if (threadIdx.x < classes) h.rows[threadIdx.x] = head->rows[threadIdx.x];
     __syncthreads();
+    if (threadIdx.x == 0) {
+        int items = 0, rows = 0;
+        for (int k = 0; k < classes; ++k) {
+            const int per = 32 >> class_shift(k % 3);
+            h.item[k] = items;
+            h.row[k] = rows;
+            items += (h.rows[k] + per - 1) / per;
+            rows += h.rows[k];
+        }
+        h.item[classes] = items;
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x <= classes) head->item[threadIdx.x] = h.item[threadIdx.x];
     unsigned long long sum = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.item[3 * kRowsWindows]; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.item[classes]; i += gridDim.x * blockDim.x) {
         int k = 0;
         while (i >= h.item[k + 1]) ++k;
         const int gs = class_shift(k % 3), per = 32 >> gs;
@@ -322,7 +325,7 @@ void RowsPlan::release() {
 }
 
 int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const double* val, int nor, long long nnz,
-               bool narrow, int sm_count, cudaStream_t st) {
+               bool narrow, int sm_count, Scratch& keep, void* pinned, cudaStream_t st) {
     R.release();
     if (nor <= 0 || nnz <= 0) return 1;
     // Lengths from which a row gets four lanes and a warp.  An item takes a
@@ -344,7 +347,8 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
     // windows from its own on, or moves up to a window with as much behind it.
     cut.up = (int)std::max(1LL, nnz / (2000LL * cut.windows));
     cut.first = kRowsLate + (int)(nnz / 32000);
-    RowsHead h{};
+    static_assert(sizeof(RowsHead) <= kPinnedBlock, "the pinned block");
+    RowsHead& h = *static_cast<RowsHead*>(pinned);
     auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
     const long long most = (long long)nor + 3 * kRowsWindows;  // items at most
     const long long tabn = triplet_sort_table_elems(nor);
@@ -354,10 +358,12 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
                  cb = up(sizeof(int32_t) * (size_t)scan_scratch_elems(std::max(tabn, most))),
                  ib = sizeof(int4) * (size_t)most;
     const int blocks = std::min(16 * sm_count, (nor + 255) / 256);
+    // past this the longest row is too long (see below)
+    const double longest = 1024.0 + std::min((double)nnz / 1000.0, 4096.0 + (double)nnz / 4000.0);
     unsigned char* tmp = nullptr;
     int rc = 2;
     do {
-        if (dev_alloc((void**)&tmp, hb + ob + 2 * kb + 2 * sb + tb + cb + ib) != cudaSuccess) break;
+        if (keep.alloc(&tmp, hb + ob + 2 * kb + 2 * sb + tb + cb + ib) != cudaSuccess) break;
         unsigned char* p = tmp;
         RowsHead* dh = reinterpret_cast<RowsHead*>(p);
         auto* off = reinterpret_cast<int32_t*>(p += hb);
@@ -371,12 +377,21 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
         if (cudaMemsetAsync(tmp, 0, hb + ob, st) != cudaSuccess) break;
         if (cut.windows > 1) std::swap(perm, other);
         k_rows_keys<<<blocks, 256, 0, st>>>(row_start, nor, cut, ka, other, dh);
+        if (cut.windows > 1) {
+            // (many rows: no sort of a matrix that a long row rules out, 1 ms on 4 M rows)
+            if (cudaMemcpyAsync(&h.longest, &dh->longest, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                break;
+            if ((double)h.longest > longest) {
+                rc = 1;
+                break;
+            }
+        }
         if (launch_radix_pass(ka, other, nor, 0, tab, scratch, kbuf, perm, st) != cudaSuccess) break;
         if (cut.windows > 1) {
             if (launch_radix_pass(kbuf, perm, nor, 8, tab, scratch, ka, other, st) != cudaSuccess) break;
             std::swap(perm, other);
         }
-        k_rows_segs<<<1, 1, 0, st>>>(dh);
         k_rows_items<<<std::min(4 * sm_count, (nor + 255) / 256), 256, 0, st>>>(row_start, perm, dh, rec, off);
         if (launch_inclusive_scan(off + 1, most, scratch, st) != cudaSuccess) break;
         if (cudaMemcpyAsync(&h, dh, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess) break;
@@ -389,8 +404,7 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
         // ones: 60 000 elements in 67 M 450 us, 560 where the row came last,
         // merge path 351; 17 000 in 16.7 M 134 and 102; eight of 10 000 in 9.5 M
         // 85 and 66.)  Padding: as the merge layout's extra.
-        if ((double)h.longest > 1024.0 + std::min((double)nnz / 1000.0, 4096.0 + (double)nnz / 4000.0) ||
-            h.units >= (1ull << 31) ||
+        if ((double)h.longest > longest || h.units >= (1ull << 31) ||
             (double)h.units * 64.0 > 1.25 * (double)nnz + 16384.0) {
             rc = 1;
             break;
@@ -426,7 +440,7 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
             break;
         k_rows_fill<<<std::min(32 * sm_count, (items + 7) / 8), 256, 0, st>>>(row_start, col, val, R.perm, items, off,
                                                                               R.rec, R.col, R.val64);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) break;
+        if (cudaGetLastError() != cudaSuccess) break;
         R.nitems = items;
         R.windows = cut.windows;
         R.wrows = cut.wrows;
@@ -434,10 +448,9 @@ int rows_build(RowsPlan& R, const int32_t* row_start, const int32_t* col, const 
         for (int w = 0; w <= kRowsWindows; ++w) R.win[w] = h.item[3 * w];
         rc = 0;
     } while (0);
-    (void)cudaStreamSynchronize(st);
-    dev_free(tmp);
     if (rc) {
         (void)cudaGetLastError();
+        if (R.mem) (void)cudaStreamSynchronize(st);
         R.release();
     }
     return rc;
