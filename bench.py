@@ -1,10 +1,10 @@
-"""Benchmark: FP64 merge-path SpMV and power method on the 4096x4096-grid
-2D Poisson matrix (N = 16,777,216, nnz = 83,869,696), GB300.
+"""Benchmark: FP64 SpMV and power method on the 4096x4096-grid 2D Poisson matrix (N = 16,777,216, nnz = 83,869,696), GB300.
 
-One step = one SpMV y = A x over the whole matrix (the plain FP64
-merge-path SpMV, reported as GB/s against the HBM roofline).  Inputs are
-larger than L2 (1.34 GB of matrix and vectors per pass), so no flush is
-needed between steps.
+One step = one SpMV y = A x over the whole matrix, in the layout its load
+chose (diagonal slices here).  value: bytes of the CRS arrays and vectors per
+second, the unit of the reference's figures; roofline: the bytes that layout has
+to stream against the HBM rate.  Inputs are larger than L2 (0.94 GB of values
+and vectors per pass), so no flush is needed between steps.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -39,6 +39,22 @@ def algorithmic_bytes(N, nnz, vbytes=8, xbytes=8):
     """12 B per nonzero (value + int32 column), int32 row_start, x read once,
     y written once."""
     return (vbytes + 4) * nnz + 4 * (N + 1) + xbytes * N + xbytes * N
+
+
+# Per layout: the kernels of an SpMV, and the bytes a nonzero streams (values
+# and, where there are any, column indices: merge sub-tiles have 2- or 4-byte
+# ones and 4 bytes per row beside).
+KERNELS = {"merge": "k_merge_spmv + k_fix_runs", "diagonals": "k_diag_spmv", "rows": "k_rows_spmv"}
+
+
+def layout_bytes(M, N, nnz):
+    """Bytes an FP64 SpMV has to stream in the layout the handle runs on."""
+    layout = M.layout()
+    if layout == "diagonals":
+        return 8 * nnz + 16 * N
+    if layout == "rows":
+        return 12 * nnz + 16 * N
+    return (8 + M.plan_info()[0]) * nnz + 4 * (N + 1) + 16 * N
 
 
 def measured_peaks():
@@ -443,7 +459,7 @@ def seeded_uniform(n, seed):
 
 
 def _one_at_a_time(pwm, kind, kw, max_it, tol):
-    """The plain FP64 merge-path path on one request: a fresh handle, the
+    """The plain FP64 path on one request: a fresh handle, the
     matrix built on the device, pwmgpu_solve.  Returns (SolveInfo,
     eigenvector)."""
     M = pwm.CRSCuda(1)
@@ -550,7 +566,7 @@ def _service_batch(pwm, S, specs, prec, max_it, tol, check):
 def serving(pwm, args):
     """Batch (256 uneven matrices) and serving-stream workloads: the batched
     service in mixed precision and in FP64 (one launch per power step for all
-    live solves, graph-captured rounds) against the plain FP64 merge-path
+    live solves, graph-captured rounds) against the plain FP64
     path solving one request at a time (pwmgpu_solve per matrix).  Every
     figure is split by matrix class (Poisson grids, random matrices); solves
     that reach the 1e-10 residual are counted apart from solves stopped at the
@@ -745,7 +761,7 @@ def triplet_load(pwm, torch, dev, M, N, cpu=True):
     same = bool(np.array_equal(trs, rs) and np.array_equal(tci, ci) and np.array_equal(tv, v))
     ms = 1e3 * sorted(times)[1]
     out = {"workload": "%d shuffled triplets of the Poisson matrix above" % nnz,
-           "api": "pwmgpu_load_triplets_device (includes the merge-path plan build)",
+           "api": "pwmgpu_load_triplets_device (includes the build of the plan and slices)",
            "ms": round(ms, 3), "entries_per_s": round(nnz / (ms * 1e-3), 1), "same_crs_as_generated": same}
     del dr, dc, dv, T
     if cpu:
@@ -934,29 +950,32 @@ def run_ours(args, world, rank, local):
         extra = dict(extra or {}, **serving(pwm, args))
 
     peak, peak_kind = measured_peaks()
-    traffic = profile_traffic().get("k_merge_spmv_f64_poisson4096")
+    layout, LB = M.layout(), layout_bytes(M, N, nnz)
+    spmv_kernels = KERNELS[layout]
+    launches = len(spmv_kernels.split(" + "))
+    traffic = profile_traffic().get("%s_f64_poisson%d" % (spmv_kernels.split(" + ")[0], grid_side))
     result = {
         "metric": METRIC, "value": round(value, 3), "unit": "GB/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms, 5), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": "poisson2d_%dx%d_fp64_spmv" % (grid_side, grid_side), "N": N, "nnz": nnz,
-                   "l2": "inputs larger than L2 (1.34 GB per pass)", "items_per_tile": tm, "tiles": ntiles,
-                   "grid": grid, "launch_variant": dict(zip(("prefer_l1", "grid", "power_grid", "tuned_ms"),
-                                                            M.launch_config()),
-                                                        column_bytes=M.plan_info()[0],
-                                                        gathers_bypass_l1=M.plan_info()[1]),
+                   "l2": "inputs larger than L2 (%.2f GB per pass)" % (LB / 1e9), "layout": layout,
+                   "merge_plan": dict(zip(("prefer_l1", "grid", "power_grid", "tuned_ms"), M.launch_config()),
+                                      items_per_tile=tm, tiles=ntiles, column_bytes=M.plan_info()[0],
+                                      gathers_bypass_l1=M.plan_info()[1]),
                    "parallelism": "replicas" if world > 1 else "single"},
-        "roofline": {"bound": "hbm", "achieved": round(B / (ms * 1e-3) / 1e9, 2), "peak": peak, "unit": "GB/s",
-                     "frac": round(B / (ms * 1e-3) / 1e9 / peak, 4), "traffic": traffic,
-                     "peak_source": peak_kind, "frac_of_nominal_8TBs": round(B / (ms * 1e-3) / 1e9 / NOMINAL_HBM_GBS, 4),
-                     "algorithmic_bytes_per_launch": B, "timed": "k_merge_spmv + k_fix_runs (one SpMV)"},
+        "roofline": {"bound": "hbm", "achieved": round(LB / (ms * 1e-3) / 1e9, 2), "peak": peak, "unit": "GB/s",
+                     "frac": round(LB / (ms * 1e-3) / 1e9 / peak, 4), "traffic": traffic,
+                     "peak_source": peak_kind, "frac_of_nominal_8TBs": round(LB / (ms * 1e-3) / 1e9 / NOMINAL_HBM_GBS, 4),
+                     "algorithmic_bytes_per_launch": LB, "crs_bytes_per_launch": B,
+                     "timed": spmv_kernels + " (one SpMV)"},
         "gflop_s": round(2.0 * nnz * world / (ms * 1e-3) / 1e9, 2),
         "e2e": ({"value": round(e2e_gbs, 3), "unit": "GB/s", "h2d_bytes_per_step": 8 * N,
                  "d2h_bytes_per_step": 8 * N, "ms_per_step": round(e2e_s * 1e3, 4),
                  "api": "pwmgpu_mv (host arrays, pinned)",
                  "pageable": {"ms_per_step": round(e2e_pageable_s * 1e3, 4),
                               "gb_s": round(B * world / e2e_pageable_s / 1e9, 3)}} if e2e_steps else None),
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": launches * args.steps,
         "power": {"iterations": p_it,
                   "fused": {"ms_per_iteration": round(power_ms["fused"] / p_it, 5),
                             "gb_s": round(B / (power_ms["fused"] / p_it * 1e-3) / 1e9, 2),
@@ -964,9 +983,8 @@ def run_ours(args, world, rank, local):
                                        "fix-up pass, barrier per iteration)"},
                   "multi": {"ms_per_iteration": round(power_ms["multi"] / p_it, 5),
                             "gb_s": round(B / (power_ms["multi"] / p_it * 1e-3) / 1e9, 2),
-                            "kernels": "k_merge_spmv + k_fix_runs per iteration (the rescale from the "
-                                       "largest magnitude key; the last two iterations sum ||y||^2 in the "
-                                       "same two kernels)"}},
+                            "kernels": spmv_kernels + " per iteration (the rescale from the largest magnitude "
+                                       "key; the last two iterations sum ||y||^2 in the same kernels)"}},
         "clocks": clk.summary(),
     }
     if formats:
