@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) k_diag_fill(const int32_t* __restrict__ r
 }
 
 // out[p] = the largest column that slices [0, ns (p + 1) / K) may read (by
-// slice and offset: up to 127 columns too many where the last rows lack it).
+// slice and offset: up to kDiagRows - 1 columns too many where the last rows lack it).
 __global__ void __launch_bounds__(256) k_diag_maxcol(const int2* __restrict__ rec, const int32_t* __restrict__ offs,
                                                      int nslices, int nor, int noc, int K, int* __restrict__ out) {
     __shared__ int red[8];
@@ -201,7 +201,7 @@ struct DiagArgs {
     const int32_t* offs;
     const unsigned* masks;  // kDiagR words per slot
     const VT* val;
-    int nor, noc, c0, c1;  // slices [c0, c1)
+    int nor, c0, c1;  // slices [c0, c1)
     const XT* x;
     XT* y;
     const unsigned int* mx_in;  // MODE_POWER / MODE_SCALE: the rescale's source (or nsq_in, or neither: e = 0)
@@ -458,23 +458,24 @@ cudaError_t launch_diag_maxcol(const DiagPlan& D, int nor, int noc, int K, int* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, int noc, const void* x, void* y,
+cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, const void* x, void* y,
                              const SliceStep& s, int sm_count, cudaStream_t st) {
     const int c1 = s.c1 < 0 ? D.nslices : s.c1;
     double* np = s.nsq_out ? D.npart : nullptr;
+    const unsigned* masks = (const unsigned*)D.masks;
     if (cfg == kCfgF64)
         return diag_mode(mode,
-                         DiagArgs<double, double>{D.rec, D.offs, (const unsigned*)D.masks, D.val64, nor, noc, s.c0, c1, (const double*)x,
+                         DiagArgs<double, double>{D.rec, D.offs, masks, D.val64, nor, s.c0, c1, (const double*)x,
                                                   (double*)y, s.mx_in, s.nsq_in, s.mx_out, np, s.counter, s.nsq_out},
                          sm_count, s.pdl, st);
     if (cfg == kCfgBF16)
         return diag_mode(mode,
-                         DiagArgs<__nv_bfloat16, float>{D.rec, D.offs, (const unsigned*)D.masks, (const __nv_bfloat16*)D.valbf, nor, noc,
-                                                        s.c0, c1, (const float*)x, (float*)y, s.mx_in, s.nsq_in,
-                                                        s.mx_out, np, s.counter, s.nsq_out},
+                         DiagArgs<__nv_bfloat16, float>{D.rec, D.offs, masks, (const __nv_bfloat16*)D.valbf, nor, s.c0,
+                                                        c1, (const float*)x, (float*)y, s.mx_in, s.nsq_in, s.mx_out,
+                                                        np, s.counter, s.nsq_out},
                          sm_count, s.pdl, st);
     return diag_mode(mode,
-                     DiagArgs<float, float>{D.rec, D.offs, (const unsigned*)D.masks, D.val32, nor, noc, s.c0, c1, (const float*)x, (float*)y,
+                     DiagArgs<float, float>{D.rec, D.offs, masks, D.val32, nor, s.c0, c1, (const float*)x, (float*)y,
                                             s.mx_in, s.nsq_in, s.mx_out, np, s.counter, s.nsq_out},
                      sm_count, s.pdl, st);
 }

@@ -196,7 +196,7 @@ struct SliceStep {
     int c0 = 0, c1 = -1;
     bool pdl = true;
 };
-cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, int noc, const void* x, void* y,
+cudaError_t launch_diag_spmv(const DiagPlan& D, int cfg, int mode, int nor, const void* x, void* y,
                              const SliceStep& s, int sm_count, cudaStream_t st);
 // Pipelined host-array SpMV: out[p] = the largest column the slices of chunks
 // 0..p read (slices [0, nslices (p + 1) / K)).

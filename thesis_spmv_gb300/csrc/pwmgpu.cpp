@@ -209,7 +209,9 @@ int tune(pwmgpu_matrix* m) {
     // A matrix on slices runs the merge kernels only where the handle asks for
     // them: two timed runs over a quarter of the sub-tiles do (at least two
     // waves of CTAs).  Load of a 2048^2 stencil: 2.67 ms with two runs over
-    // all of them, 2.18 so (the same variants chosen, stencils and irregular).
+    // all of them, 2.18 so (stencils and irregular matrices chose the same
+    // variants, but for one of three loads of a 1 M-row one, whose variants 1
+    // and 5 lie within 0.2 % of each other).
     const bool side = sliced(m);
     const int reps = side ? 2 : 8, tiles = side ? m->num_tiles / 4 : m->num_tiles;
     for (int c = 0; c < 4 && rc == PWMGPU_OK; ++c) {
@@ -486,7 +488,7 @@ int fp64_format(const pwmgpu_matrix* m) {
 }
 
 cudaError_t launch_sliced(pwmgpu_matrix* m, int cfg, int mode, const void* x, void* y, const SliceStep& s) {
-    return m->diag.nslices ? launch_diag_spmv(m->diag, cfg, mode, m->M.nor, m->M.noc, x, y, s, m->sm_count, m->stream)
+    return m->diag.nslices ? launch_diag_spmv(m->diag, cfg, mode, m->M.nor, x, y, s, m->sm_count, m->stream)
                            : launch_rows_spmv(m->rows, cfg, mode, x, y, s, m->stream);
 }
 
@@ -571,10 +573,10 @@ int scale_step_f64(pwmgpu_matrix* m, const double* in, double* out, const double
     return PWMGPU_OK;
 }
 
-// POWER_AUTO runs the two-kernel step at every size: its kernel boundaries
-// (programmatic dependent launch) cost less than the persistent kernel's
-// grid barriers, and its SpMV keeps the most resident CTAs.  Per iteration,
-// Poisson grids: 256^2 6.5 vs 11.0 us, 512^2 10.7 vs 19.7 us, 1024^2 21.7 vs
+// POWER_AUTO runs a step of one kernel on slices and of two (SpMV, fix-up) on
+// the merge plan, at every size: kernel boundaries (programmatic dependent
+// launch) cost less than the persistent kernel's grid barriers, and the SpMV
+// keeps the most resident CTAs.  Merge plan, per iteration, Poisson grids: 256^2 6.5 vs 11.0 us, 512^2 10.7 vs 19.7 us, 1024^2 21.7 vs
 // 30.4 us, 2048^2 63.2 vs 72.3 us, 4096^2 0.223 vs 0.240 ms; the irregular 4M
 // matrix 0.393 vs 0.425 ms.  POWER_FUSED selects the persistent kernel.
 bool use_fused(const pwmgpu_matrix* m, int pgrid) {
