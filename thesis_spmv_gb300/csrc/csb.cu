@@ -61,14 +61,17 @@ namespace {
 
 // Kernel variants (launch_csb_spmv's `variant`): bit 0 = 8 elements of a
 // dense unit per lane (else 4), bit 1 = 256 threads per CTA (else 128).
-// Resident CTAs per SM (24.6 KB of shared memory each): 7 of 128 threads, 4
-// of 256.  The loads in flight land in what shared memory leaves of L1, and
-// they bound a stencil: 4096^2 Poisson 227 us at 7 CTAs of 128
-// (about 4 % more at 6, 20 % at 8); 277 at 8 before a unit's elements were loaded at once and
-// diagonals of a tile shared an x window.  The random 1 M row matrix: 111 us
-// at 4 CTAs of 256, 122 at 3.  Variant 0 is the default; the format autotuner times all
-// four.
-constexpr int csb_ctas(int nt) { return nt == 128 ? 7 : 4; }
+// Variant 0 is the default; the format autotuner times all four.
+//
+// Resident CTAs per SM (24.6 KB of shared memory each): 7 of 128 threads, 4 of
+// 256.  The loads in flight land in what shared memory leaves of L1, and they
+// bound a stencil (4096^2 Poisson 227 us at 7 CTAs of 128, about 4 % more at 6,
+// 20 % at 8) and an irregular matrix (1 M rows of 8: 77 us, 104 at 8).  Resident
+// CTAs stride over the windows, so what counts on 1000 to 4000 windows is the
+// rounds: 8 CTAs (fewer registers) where they save one and a round of theirs,
+// 1.3 times as long, costs less than it (290 000-row stencil, 1133 windows 16.4
+// us at 8 and 18.5 at 7; 1.15 M irregular rows, 2247 windows 148 and 182).
+constexpr int kCsbRoundCost = 13;  // tenths
 constexpr int kCsbMaxS = 1024;
 constexpr int kDenseUnit = kTileDenseUnit;  // elements from which a unit's x window is staged
 
@@ -262,8 +265,10 @@ __device__ __forceinline__ void dense_oct(const Oct<K>& q, int S, const double* 
 
 // win_ptr[2w] = the window's first unit, win_ptr[2w+1] = its first dense
 // unit, win_ptr[2w+2] = the next window's first unit.
-template <int NT, int K>
-__global__ void __launch_bounds__(NT, csb_ctas(NT)) k_csb_spmv(const uint32_t* __restrict__ ind, const int32_t* __restrict__ kcol, const double* __restrict__ data,
+// CTAS: resident CTAs per SM; U: elements of a one-per-row unit that a lane
+// loads at once; STREAM: windows of kCsbMaxS rows (see launch_csb_spmv).
+template <int NT, int K, int CTAS, int U, bool STREAM>
+__global__ void __launch_bounds__(NT, CTAS) k_csb_spmv(const uint32_t* __restrict__ ind, const int32_t* __restrict__ kcol, const double* __restrict__ data,
                                                      const int* __restrict__ win_ptr, const int4* __restrict__ units,
                                                      int nwin, int S, int nor, int noc, const double* __restrict__ x,
                                                      double* __restrict__ y, const double* nsq_in, int* status) {
@@ -316,15 +321,17 @@ __global__ void __launch_bounds__(NT, csb_ctas(NT)) k_csb_spmv(const uint32_t* _
         bool ok = true;
         for (int u = u0; u < u1; ++u) {
             const int4 un = __ldg(units + u);
-            // a new x window (diagonals of one tile share theirs)
-            const bool fresh = u == u0 || __ldg(&units[u - 1].z) != un.z;
+            // a new x window (diagonals of one tile share theirs; looking for
+            // it costs more than it saves where windows are small)
+            const bool fresh = !STREAM || u == u0 || __ldg(&units[u - 1].z) != un.z;
             // ys holds the units before; the x window before is free, so the
             // next one lands there
             auto turn = [&]() {
                 __syncthreads();
                 if (!fresh) return;
                 int ahead = u + 1;
-                while (ahead < u1 && __ldg(&units[ahead].z) == un.z) ++ahead;
+                if (STREAM)
+                    while (ahead < u1 && __ldg(&units[ahead].z) == un.z) ++ahead;
                 if (ahead < u1) stage(ahead, (n + 1) & 1);
             };
             auto landed = [&]() {
@@ -335,33 +342,58 @@ __global__ void __launch_bounds__(NT, csb_ctas(NT)) k_csb_spmv(const uint32_t* _
                 return ok;
             };
             if (un.w == 2) {
-                // one element per row (at most S of them): element lo + i to
-                // lane i % 32 of a warp, so a warp's loads, x-window reads and
-                // y-window updates are 32 consecutive rows (no bank
-                // conflicts), U per lane in flight while the x window lands;
-                // one FMA per element from the row's y-window value
-                constexpr int U = kCsbMaxS / NT;
+                // one element per row: 32 consecutive ones to a warp, so its
+                // loads, x-window reads and y-window updates are of 32
+                // consecutive rows (no bank conflicts), U per lane in flight
+                // while the x window lands; one FMA per element from the row's
+                // y-window value.  A warp's U loads lie side by side where the
+                // CTA takes a whole window's unit with 8 (4096^2 Poisson 227
+                // us, 242 the other way), else NT apart, so that a short unit
+                // has all warps.
+                constexpr int STEP = U == 8 ? 32 : NT;
                 uint32_t id[U];
-                double v[U], acc[U];
-                const int k0 = un.x + warp * (32 * U) + lane;
+                double v[U];
+                int k0 = un.x + (STEP == 32 ? warp * (32 * U) + lane : tid);
+                auto load = [&]() {
 #pragma unroll
-                for (int t = 0; t < U; ++t) {
-                    const bool in = k0 + 32 * t < un.y;
-                    id[t] = in ? __ldcs(ind + k0 + 32 * t) : 0u;
-                    v[t] = in ? __ldcs(data + k0 + 32 * t) : 0.0;
-                }
+                    for (int t = 0; t < U; ++t) {
+                        const bool in = k0 + STEP * t < un.y;
+                        id[t] = !in ? 0u : STREAM ? __ldcs(ind + k0 + STEP * t) : __ldg(ind + k0 + STEP * t);
+                        v[t] = !in ? 0.0 : STREAM ? __ldcs(data + k0 + STEP * t) : __ldg(data + k0 + STEP * t);
+                    }
+                };
+                load();
                 turn();
                 if (!landed()) break;
                 const double* xw = xs[(n - 1) & 1];
+                for (;;) {
+                    if (K == 8 && !STREAM) {
+                        // (8 elements of a dense unit leave no registers for
+                        // the U sums: with them the loop spills, 1.15 M
+                        // irregular rows 154 us, so 144)
 #pragma unroll
-                for (int t = 0; t < U; ++t)
-                    if (k0 + 32 * t < un.y) acc[t] = ys[(int)(id[t] >> 16) & (S - 1)];
+                        for (int t = 0; t < U; ++t)
+                            if (k0 + STEP * t < un.y) {
+                                double& s = ys[(int)(id[t] >> 16) & (S - 1)];
+                                s = fma(v[t], xw[id[t] & (uint32_t)(S - 1)], s);
+                            }
+                    } else {
+                        double acc[U];
 #pragma unroll
-                for (int t = 0; t < U; ++t)
-                    if (k0 + 32 * t < un.y) acc[t] = fma(v[t], xw[id[t] & (uint32_t)(S - 1)], acc[t]);
+                        for (int t = 0; t < U; ++t)
+                            if (k0 + STEP * t < un.y) acc[t] = ys[(int)(id[t] >> 16) & (S - 1)];
 #pragma unroll
-                for (int t = 0; t < U; ++t)
-                    if (k0 + 32 * t < un.y) ys[(int)(id[t] >> 16) & (S - 1)] = acc[t];
+                        for (int t = 0; t < U; ++t)
+                            if (k0 + STEP * t < un.y) acc[t] = fma(v[t], xw[id[t] & (uint32_t)(S - 1)], acc[t]);
+#pragma unroll
+                        for (int t = 0; t < U; ++t)
+                            if (k0 + STEP * t < un.y) ys[(int)(id[t] >> 16) & (S - 1)] = acc[t];
+                    }
+                    if (NT * U >= kCsbMaxS) break;  // the unit has at most S elements
+                    k0 += NT * U;
+                    if (k0 - tid >= un.y) break;
+                    load();
+                }
                 continue;
             }
             // row-major unit: warp chunks of kChunk elements; the first
@@ -689,16 +721,30 @@ cudaError_t launch_csb_spmv(const uint32_t* ind, const int32_t* kcol, const doub
     if (nwin <= 0) return cudaSuccess;
     const int4* un = reinterpret_cast<const int4*>(units);
     const int nt = (variant & 2) ? 256 : 128;
+    // Windows of 1024 rows hold a matrix larger than L2 (1.2 M rows and more):
+    // streamed, and at 7 CTAs of 128 threads 8 elements of a lane at once (4096^2
+    // Poisson 227 us, 255 with 4).  Smaller windows have fewer elements than
+    // that per lane (560 000-row stencil 27 us with 8, 18.6 with 4), and L2
+    // keeps them for the next product (18.6 us, 20.6 streamed).
+    const bool stream = S == kCsbMaxS;
     // 256 threads (irregular matrices): a CTA per window, so the block
     // scheduler evens out windows of unequal work (random 1 M rows: 111 us,
     // 114 with resident CTAs that stride over the windows); 128 threads
     // (stencils, equal windows): resident CTAs (4096^2 Poisson 227 us, 231).
-    const int grid = nt == 256 ? nwin : std::min(nwin, sm_count * csb_ctas(nt));
-    switch (variant & 3) {
-        case 1: k_csb_spmv<128, 8><<<grid, 128, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
-        case 2: k_csb_spmv<256, 4><<<grid, 256, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
-        case 3: k_csb_spmv<256, 8><<<grid, 256, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
-        default: k_csb_spmv<128, 4><<<grid, 128, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status); break;
+    const auto rounds = [&](int ctas) { return (nwin + ctas * sm_count - 1) / (ctas * sm_count); };
+    const bool eight = kCsbRoundCost * rounds(8) < 10 * rounds(7);
+    const int grid = nt == 256 ? nwin : std::min(nwin, (eight ? 8 : 7) * sm_count);
+    const auto run = [&](auto* kernel) {
+        kernel<<<grid, nt, 0, st>>>(ind, kcol, data, win_ptr, un, nwin, S, nor, noc, x, y, nsq_in, status);
+    };
+    if (variant & 1) {
+        if (nt == 256) stream ? run(k_csb_spmv<256, 8, 4, 4, true>) : run(k_csb_spmv<256, 8, 4, 4, false>);
+        else if (eight) stream ? run(k_csb_spmv<128, 8, 8, 4, true>) : run(k_csb_spmv<128, 8, 8, 4, false>);
+        else stream ? run(k_csb_spmv<128, 8, 7, 8, true>) : run(k_csb_spmv<128, 8, 7, 4, false>);
+    } else {
+        if (nt == 256) stream ? run(k_csb_spmv<256, 4, 4, 4, true>) : run(k_csb_spmv<256, 4, 4, 4, false>);
+        else if (eight) stream ? run(k_csb_spmv<128, 4, 8, 4, true>) : run(k_csb_spmv<128, 4, 8, 4, false>);
+        else stream ? run(k_csb_spmv<128, 4, 7, 8, true>) : run(k_csb_spmv<128, 4, 7, 4, false>);
     }
     return cudaGetLastError();
 }
