@@ -29,8 +29,8 @@
 // Measured against the layouts it replaced, y = A x (GB300): FP64 4096^2
 // 5-point 0.208 -> 0.160 ms, 3001 x 2777 5-point 0.105 -> 0.080, 1999 x 1501
 // 9-point 0.073 -> 0.061, 512^2 9.4 -> 4.9 us; FP32 4096^2 0.151 -> 0.091 ms,
-// 1999 x 1501 9-point 0.045 -> 0.022; power step 4096^2 0.217 -> 0.167 ms,
-// 512^2 11.1 -> 6.3 us.
+// 1999 x 1501 9-point 0.046 -> 0.025; power step 4096^2 0.217 -> 0.164 ms,
+// 512^2 11.1 -> 6.2 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
