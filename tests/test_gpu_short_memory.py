@@ -19,6 +19,15 @@ def leave(gb):
     torch.cuda.synchronize()
     free = torch.cuda.mem_get_info()[0]
     return torch.empty(free - int(gb * (1 << 30)), dtype=torch.uint8, device="cuda")
+def fill():
+    # what the library still finds, also in its own pool
+    out = []
+    try:
+        while True:
+            out.append(pwm.CRSCuda(1))
+            out[-1].generatePoissonMatrix(1024, 1024, 1)
+    except RuntimeError:
+        return out
 def check(m):
     n = m * m
     x = np.random.default_rng(1).random(n).reshape(m, m)
@@ -87,3 +96,34 @@ for _ in range(3):
     M.generatePoissonMatrix(2048, 2048, 1)
     check(2048)
 """)
+
+
+@pytest.mark.parametrize("then", ["the same product", "a small product"])
+def test_vectors_that_do_not_fit(then):
+    """The load fits, the vectors of a host-array product (0.37 GiB each: ten rows
+    of 50 M columns) do not: an error, and the handle's next products have
+    vectors again."""
+    _run("""
+check(8)
+def wide():
+    M.loadCSR(10, 50_000_000, np.arange(11, dtype=np.int32), np.arange(10, dtype=np.int32) * 4_999_999, np.ones(10))
+def product():
+    x, y = np.arange(50_000_000) % 1000 * 1.0, np.full(10, np.nan)
+    M.mv(x, y)
+    assert np.array_equal(y, x[np.arange(10) * 4_999_999])
+wide()
+hog = leave(0.15)
+others = fill()
+try:
+    product()
+    raise SystemExit("the vectors should not have fitted")
+except RuntimeError:
+    pass
+""" + ("""
+del others, hog
+torch.cuda.empty_cache()
+product()
+""" if then == "the same product" else """
+M.generatePoissonMatrix(8, 8, 1)
+check(8)
+"""))

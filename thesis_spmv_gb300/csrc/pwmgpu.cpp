@@ -406,6 +406,7 @@ int ensure_vectors(pwmgpu_matrix* m) {
     size_t need = (size_t)std::max(m->M.nor, m->M.noc) + kPad;
     if (m->vec_cap >= need) return PWMGPU_OK;
     size_t cx = m->vec_cap, cy = m->vec_cap;
+    m->vec_cap = 0;  // (one of them may be gone where the other does not fit)
     TRY(ensure_cap(m, &m->dx, &cx, need));
     TRY(ensure_cap(m, &m->dy, &cy, need));
     m->vec_cap = std::min(cx, cy);
@@ -748,6 +749,7 @@ int ensure_fvectors(pwmgpu_matrix* m) {
     size_t need = (size_t)std::max(m->M.nor, m->M.noc) + kPad;
     if (m->fvec_cap >= need) return PWMGPU_OK;
     size_t cx = m->fvec_cap, cy = m->fvec_cap;
+    m->fvec_cap = 0;
     TRY(ensure_cap(m, &m->fx, &cx, need));
     TRY(ensure_cap(m, &m->fy, &cy, need));
     m->fvec_cap = std::min(cx, cy);
