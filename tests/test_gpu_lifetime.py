@@ -151,3 +151,31 @@ def test_one_small_handle_after_another():
     r = subprocess.run([sys.executable, "-c", LONE], capture_output=True, text=True, timeout=300,
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+def test_a_handle_dropped_beside_a_relaxed_capture():
+    """A relaxed capture on a stream allows frees elsewhere: another handle made,
+    loaded and dropped meanwhile, and the replays give the product."""
+    torch = pytest.importorskip("torch")
+    import thesis_spmv_gb300 as pwm
+    M = pwm.CRSCuda(1)
+    M.generatePoissonMatrix(300, 200, 1)
+    n = M.dims()[0]
+    x = torch.rand(n, dtype=torch.float64, device="cuda")
+    want, y = torch.empty_like(x), torch.zeros_like(x)
+    torch.cuda.synchronize()
+    M.mv_device(x.data_ptr(), want.data_ptr())
+    torch.cuda.synchronize()
+    N = pwm.CRSCuda(1)
+    N.generatePoissonMatrix(300, 200, 1)
+    s = torch.cuda.Stream()
+    M.set_stream(s.cuda_stream)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="relaxed"):
+        M.mv_device(x.data_ptr(), y.data_ptr())
+        N.generatePoissonMatrix(70, 80, 1)
+        del N
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    M.set_stream(0)

@@ -52,7 +52,7 @@ cudaError_t dev_alloc(void** out, size_t bytes);
 void dev_free(void* p);
 // Waits for all work on `device` (as cudaFree does), so that blocks whose users
 // are not all known can be freed inside the scope.  Where the wait is refused
-// (a stream is being captured), the scope's dev_free calls keep their blocks
+// (a stream is being captured, not relaxed), the scope's dev_free calls keep their blocks
 // until a later scope's wait succeeds.
 class DevIdle {
 public:
