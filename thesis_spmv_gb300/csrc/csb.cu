@@ -14,8 +14,8 @@
 // the block row, every column window) and adds each element's product into
 // the y window, then writes its rows of y once.  Dense units (at least
 // kDenseUnit elements) stage their S-column x window in shared memory with a
-// TMA bulk copy (double-buffered, mbarriers; units in a row with the same
-// window share it) and are taken by the whole CTA;
+// TMA bulk copy (double-buffered, mbarriers; where S is 1024, units in a row
+// with the same window share it) and are taken by the whole CTA;
 // a window's sparse units (a random matrix's blocks hold a few elements
 // each) are merged into one "flat" unit taken by the whole CTA, gathering x
 // through L1/L2 by global column -- staging 8 KB of x for a handful of
